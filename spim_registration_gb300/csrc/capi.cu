@@ -453,11 +453,16 @@ struct mvd_decon {
     std::unique_ptr<ConvPlan> ext;   // plan over the volume extended by k/2 (tiles shifted by -k/2)
     DevBuf otf_m;                    // spectrum of mirror(kernel1) on `ext`
     DevBuf fold_tab;                 // CSR tables of the mirror fold
-    DevBuf lag_tile, lag_items_z, lag_items_inv;  // one full tile of the view's plan
-    int n_lag_z = 0, n_lag_inv = 0;
+    // The residual and the PSF gradient run on the scalar kernels.  The gradient is what is left of
+    // a sum over the volume that nearly cancels (the residuals' mean is close to zero), so its
+    // FP32 rounding error is 1e-4 of it and moves with every change of the summation order.
+    std::unique_ptr<ConvPlan> scalar;  // null: the view's own plan is a scalar one
+    DevBuf otf1;                       // spectrum of kernel1 on it
   };
   std::vector<AdjView> adj;
-  DevBuf r, c_ext, spec_ext, spec_b, acc, lag_real, g_psi, g_psf, d_nll;
+  DevBuf r, c_ext, spec_ext, spec_a, spec_b, acc, lag_real, g_psi, g_psf, d_nll;
+  const ConvPlan& adj_plan(int v) const { return adj[v].scalar ? *adj[v].scalar : *plans[v]; }
+  const float2* adj_otf(int v) const { return (adj[v].scalar ? adj[v].otf1 : otf1[v]).as<float2>(); }
 
   StatSlot* slot(int v) { return stats.as<StatSlot>() + v; }
 
@@ -703,17 +708,30 @@ std::unique_ptr<ConvPlan> plan_view(mvd_decon* h, int v, const int lo[3], const 
     PlanOptions o;
     o.cap = cap;
     o.ascending = ascending;
+    o.scalar = tensor_dft;  // the tensor-core stage belongs to the scalar z pass
+    o.off_x = lo[0];
+    o.vol_x = h->dims[0];
     auto p = make_conv_plan(h->pt, n[0], n[1], n[2], k[0], k[1], k[2], o);
     if (!full) place_plan(*p, lo[0], lo[1], lo[2], h->dims);
     p->tensor_dft = tensor_dft;
     return p;
   };
   if (!autotune) return make(0, false);
+  auto make_pair = [&](int kb) {  // a pair plan whose plane buffer takes at most kb KB (0: any)
+    PlanOptions o;
+    o.pair_smem = (size_t)kb * 1024;
+    o.off_x = lo[0];
+    o.vol_x = h->dims[0];
+    auto p = make_conv_plan(h->pt, n[0], n[1], n[2], k[0], k[1], k[2], o);
+    if (!full) place_plan(*p, lo[0], lo[1], lo[2], h->dims);
+    return p;
+  };
   const std::array<int, 8> key{h->dev, n[0], n[1], n[2], k[0], k[1], k[2], tensor_dft ? 1 : 0};
   {
     std::lock_guard<std::mutex> lock(g_tuned_mu);
     auto it = g_tuned.find(key);
     if (it != g_tuned.end()) {
+      if (use_pairs() && !tensor_dft && it->second.threads == 0) return make_pair(it->second.cap);
       auto p = make(it->second.cap, it->second.ascending);
       p->threads_plane = it->second.threads;
       p->generic = it->second.generic || it->second.ascending;
@@ -743,6 +761,41 @@ std::unique_ptr<ConvPlan> plan_view(mvd_decon* h, int v, const int lo[3], const 
     }
     return ms;
   };
+  std::vector<std::array<int, 3>> seen;
+  if (use_pairs() && !tensor_dft) {
+    // pair kernels: the default shape and the best ones with at most one, two, three and four plane
+    // CTAs per SM, each at the CTA size of its occupancy
+    std::unique_ptr<ConvPlan> best;
+    TunedChoice choice{0, 0, false, false, false};
+    float best_ms = 1e30f;
+    for (int kb : {0, 226, 112, 74, 55}) {
+      std::unique_ptr<ConvPlan> p;
+      try {
+        p = make_pair(kb);
+      } catch (const std::invalid_argument&) {
+        continue;
+      }
+      if (!p->paired) continue;  // no pair shape within this budget
+      const std::array<int, 3> shape{p->ax.T, p->ay.T, p->az.T};
+      if (std::find(seen.begin(), seen.end(), shape) != seen.end()) continue;
+      seen.push_back(shape);
+      DevBuf otf(p->otf_elems * sizeof(float2)), spec(p->spec_elems * sizeof(float2));
+      MVD_CHECK(cudaMemsetAsync(otf.p, 0, otf.bytes, h->stream));
+      const float t = time_stage(*p, otf, spec);
+      if (t < best_ms) {
+        best_ms = t;
+        choice.cap = kb;
+        best = std::move(p);
+      }
+    }
+    if (best) {
+      cudaEventDestroy(e0);
+      cudaEventDestroy(e1);
+      std::lock_guard<std::mutex> lock(g_tuned_mu);
+      g_tuned[key] = choice;
+      return best;
+    }
+  }
   // Candidates: the tile shapes of four plane budgets; for each, the default kernels (the
   // compiled ones where the shape has them), the generic kernels at 384 threads (where compiled
   // ones exist) and at 256 threads, and the generic kernels with every length's radices in
@@ -750,7 +803,7 @@ std::unique_ptr<ConvPlan> plan_view(mvd_decon* h, int v, const int lo[3], const 
   std::unique_ptr<ConvPlan> best;
   TunedChoice best_choice{0, kThreads, false, false, false};
   float best_ms = 1e30f;
-  std::vector<std::array<int, 3>> seen;
+  seen.clear();
   for (int cap : {4608, 7168, 10240, 14336}) {
     auto p = make(cap, false);
     const std::array<int, 3> shape{p->ax.T, p->ay.T, p->az.T};
@@ -1132,6 +1185,11 @@ extern "C" int mvd_get_plan_variant(mvd_decon* h, int view, int* threads, int* v
   if (!h) return fail(MVD_ERR_ARG, "NULL handle");
   if (view < 0 || view >= h->V) return fail(MVD_ERR_ARG, "view out of range");
   const ConvPlan& p = *h->plans[view];
+  if (p.paired) {
+    if (threads) *threads = p.pair_threads;
+    if (variant) *variant = 16;
+    return MVD_OK;
+  }
   const bool compiled = !p.generic && has_compiled_kernels(p) && p.threads_plane == kThreads;
   const bool staged = compiled && p.staged && has_staged_kernels(p);
   if (threads) *threads = staged ? 512 : compiled && compiled_plane_threads(p) ? compiled_plane_threads(p) : p.threads_plane;
@@ -1242,38 +1300,28 @@ void adjoint_setup(mvd_decon* h) {
     }
     a.fold_tab.alloc(tab.size() * sizeof(int));
     upload_table(a.fold_tab.p, tab.data(), tab.size() * sizeof(int));
-    // one full tile of the view's plan, for the inverse transform of the accumulated spectrum
-    const ConvPlan& p = *h->plans[v];
-    TileDesc t = p.tiles[0];
-    t.ox = t.oy = t.oz = 0;
-    t.hx = t.hy = t.hz = 0;
-    t.ex = p.ax.T;
-    t.ey = p.ay.T;
-    t.ez = p.az.T;
-    t.spec_off = 0;
-    t.otf_off = 0;
-    std::vector<int2> iz, ii;
-    for (int p0 = 0; p0 < t.ty * t.px; p0 += kZChunk) iz.push_back(make_int2(0, p0));
-    for (int z = 0; z < t.tz; ++z) ii.push_back(make_int2(0, z));
-    a.lag_tile.alloc(sizeof(TileDesc));
-    a.lag_items_z.alloc(iz.size() * sizeof(int2));
-    a.lag_items_inv.alloc(ii.size() * sizeof(int2));
-    upload_table(a.lag_tile.p, &t, sizeof(TileDesc));
-    upload_table(a.lag_items_z.p, iz.data(), iz.size() * sizeof(int2));
-    upload_table(a.lag_items_inv.p, ii.data(), ii.size() * sizeof(int2));
-    a.n_lag_z = (int)iz.size();
-    a.n_lag_inv = (int)ii.size();
+    if (h->plans[v]->paired) {
+      const ConvPlan& own = *h->plans[v];
+      PlanOptions o;
+      o.scalar = true;
+      a.scalar = make_conv_plan(h->pt, own.nx, own.ny, own.nz, k[0], k[1], k[2], o);
+      place_plan(*a.scalar, own.box_lo[0], own.box_lo[1], own.box_lo[2], h->dims);
+      a.otf1.alloc(a.scalar->otf_elems * sizeof(float2));
+      build_otf(h->pt, *a.scalar, h->k1[v].as<float>(), a.otf1.as<float2>(), h->scratch, h->stream);
+    }
+    const ConvPlan& p = h->adj_plan(v);
     tile_max = std::max(tile_max, (long long)p.ax.T * p.ay.T * p.az.T);
     otf_max = std::max(otf_max, p.otf_elems);
   }
   long long spec_max = 0, kmax = 0;
   for (int v = 0; v < h->V; ++v) {
-    spec_max = std::max(spec_max, h->plans[v]->spec_elems);
+    spec_max = std::max(spec_max, h->adj_plan(v).spec_elems);
     kmax = std::max(kmax, vox(h->kd[v]));
   }
   h->r.alloc(h->N * sizeof(float));
   h->c_ext.alloc(ext_max * sizeof(float));
   h->spec_ext.alloc(spec_ext_max * sizeof(float2));
+  h->spec_a.alloc(spec_max * sizeof(float2));
   h->spec_b.alloc(spec_max * sizeof(float2));
   h->acc.alloc(otf_max * sizeof(float2));
   h->lag_real.alloc(tile_max * sizeof(float));
@@ -1285,10 +1333,10 @@ void adjoint_setup(mvd_decon* h) {
 
 // f_v = ext(psi) (*) kernel1_v; NLL epilogue (residual into h->r when `residual`)
 void enqueue_blur_nll(mvd_decon* h, int v, bool residual) {
-  const ConvPlan& p = *h->plans[v];
-  float2* sp = h->spec.as<float2>();
+  const ConvPlan& p = residual ? h->adj_plan(v) : *h->plans[v];
+  float2* sp = (residual ? h->spec_a : h->spec).as<float2>();
   launch_fwd_mirror(h->pt, p, h->psi.as<float>(), sp, h->stream);
-  launch_z(h->pt, p, sp, h->otf1[v].as<float2>(), h->stream);
+  launch_z(h->pt, p, sp, residual ? h->adj_otf(v) : h->otf1[v].as<float2>(), h->stream);
   launch_inv_nll(h->pt, p, sp, h->img[v].as<float>(), h->w[v].as<float>(), residual ? h->r.as<float>() : nullptr,
                  h->d_nll.as<double>(), h->stream);
 }
@@ -1322,7 +1370,7 @@ extern "C" int mvd_backward(mvd_decon* h, float* grad_psi, float* const* grad_ps
   MVD_CHECK(cudaMemsetAsync(h->d_nll.p, 0, sizeof(double), s));
   MVD_CHECK(cudaMemsetAsync(h->r.p, 0, h->N * sizeof(float), s));  // zero outside the views' data boxes
   for (int v = 0; v < h->V; ++v) {
-    const ConvPlan& p = *h->plans[v];
+    const ConvPlan& p = h->adj_plan(v);
     mvd_decon::AdjView& a = h->adj[v];
     const auto& k = h->kd[v];
     // recompute this view's blur and residual (no blurred view is kept between calls)
@@ -1331,28 +1379,24 @@ extern "C" int mvd_backward(mvd_decon* h, float* grad_psi, float* const* grad_ps
     // then folded back through the mirror-single extension
     const ConvPlan& e = *a.ext;
     float2* se = h->spec_ext.as<float2>();
-    launch_fwd_value_items(h->pt, e, e.d_tiles.as<TileDesc>(), e.d_items_fwd.as<int2>(), (int)e.items_fwd.size(),
-                           h->r.as<float>(), h->dims[0], h->dims[1], h->dims[2], 0.f, se, s);
+    launch_fwd_value_tiles(h->pt, e, TileSet::All, h->r.as<float>(), h->dims[0], h->dims[1], h->dims[2], 0.f, se, s);
     launch_z(h->pt, e, se, a.otf_m.as<float2>(), s);
     const long long off = ((long long)(k[2] / 2) * e.ny + k[1] / 2) * e.nx + k[0] / 2;
-    launch_inv_store_items(h->pt, e, e.d_tiles.as<TileDesc>(), e.d_items_inv.as<int2>(), (int)e.items_inv.size(),
-                           se, h->c_ext.as<float>() + off, e.nx, e.ny, s);
+    launch_inv_store_tiles(h->pt, e, TileSet::All, se, h->c_ext.as<float>() + off, e.nx, e.ny, s);
     dev_fold_mirror(h->c_ext.as<float>(), e.nx, e.ny, a.fold_tab.as<int>(), h->dims[0], h->dims[1], h->dims[2],
                     h->g_psi.as<float>(), s);
     // dNLL/dP_v(j) = sum_x r(x) ext(psi)(x - (j - k/2)): per tile, spectrum of the residual
     // restricted to the effective region times the conjugate spectrum of ext(psi) over the
     // tile window, summed over tiles; one inverse transform; the kernel-sized lags
-    float2* sa = h->spec.as<float2>();
+    float2* sa = h->spec_a.as<float2>();
     float2* sb = h->spec_b.as<float2>();
     launch_fwd_mirror(h->pt, p, h->psi.as<float>(), sa, s);
-    launch_z_forward(h->pt, p, sa, s);
+    launch_z_forward(h->pt, p, TileSet::All, sa, 1.f, s);
     launch_fwd_masked(h->pt, p, h->r.as<float>(), sb, s);
-    launch_z_forward(h->pt, p, sb, s);
+    launch_z_forward(h->pt, p, TileSet::All, sb, 1.f, s);
     dev_cross_accumulate(sb, sa, (int)p.tiles.size(), p.otf_elems, h->acc.as<float2>(), s);
-    launch_z_inverse_items(h->pt, p, a.lag_tile.as<TileDesc>(), a.lag_items_z.as<int2>(), a.n_lag_z,
-                           h->acc.as<float2>(), s);
-    launch_inv_store_items(h->pt, p, a.lag_tile.as<TileDesc>(), a.lag_items_inv.as<int2>(), a.n_lag_inv,
-                           h->acc.as<float2>(), h->lag_real.as<float>(), p.ax.T, p.ay.T, s);
+    launch_z_inverse(h->pt, p, TileSet::Full, h->acc.as<float2>(), s);
+    launch_inv_store_tiles(h->pt, p, TileSet::Full, h->acc.as<float2>(), h->lag_real.as<float>(), p.ax.T, p.ay.T, s);
     const double n_tile = (double)p.ax.T * p.ay.T * p.az.T;
     dev_extract_lags(h->lag_real.as<float>(), p.ax.T, p.ay.T, p.az.T, k[0], k[1], k[2], (float)(1.0 / n_tile),
                      h->g_psf.as<float>(), s);
@@ -1371,6 +1415,9 @@ extern "C" int mvd_set_kernel(mvd_decon* h, int view, int which, const float* da
   MVD_CHECK(cudaSetDevice(h->dev));
   AllocScope scope(h->stream);
   DevBuf& k = which == 1 ? h->k1[view] : h->k2[view];
+  // copied from pageable memory before the call returns; from page-locked memory by the wait below.
+  // The spectra need no wait: whatever uses them runs on the handle's stream.
+  const bool async_src = async_copy_source(data);
   MVD_CHECK(cudaMemcpyAsync(k.p, data, vox(h->kd[view]) * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   const ConvPlan& p = *h->plans[view];
   build_otf(h->pt, p, k.as<float>(), (which == 1 ? h->otf1[view] : h->otf2[view]).as<float2>(), h->scratch,
@@ -1379,8 +1426,10 @@ extern "C" int mvd_set_kernel(mvd_decon* h, int view, int which, const float* da
     mvd_decon::AdjView& a = h->adj[view];
     DevBuf mk = mirrored(h, h->k1[view].as<float>(), h->kd[view]);
     build_otf(h->pt, *a.ext, mk.as<float>(), a.otf_m.as<float2>(), h->scratch, h->stream);
+    if (a.scalar)
+      build_otf(h->pt, *a.scalar, h->k1[view].as<float>(), a.otf1.as<float2>(), h->scratch, h->stream);
   }
-  MVD_CHECK(cudaStreamSynchronize(h->stream));
+  if (async_src) MVD_CHECK(cudaStreamSynchronize(h->stream));
   return MVD_OK;
   MVD_API_END
 }

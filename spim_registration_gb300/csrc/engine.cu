@@ -257,6 +257,7 @@ static void fill_items(ConvPlan& p) {
 }
 
 void ConvPlan::upload() {
+  if (paired) return upload_pair();
   d_tiles.alloc(tiles.size() * sizeof(TileDesc));
   upload_table(d_tiles.p, tiles.data(), tiles.size() * sizeof(TileDesc));
   auto up = [](DevBuf& b, const std::vector<int2>& v) {
@@ -400,11 +401,313 @@ bool use_fixed_planes() {
   return on;
 }
 
+bool use_pairs() {
+  static bool on = [] {
+    const char* e = std::getenv("MVD_PAIRED");
+    if (e && e[0] == '0') return false;
+    for (const char* v : {"MVD_FIXED_PLANES", "MVD_STAGED_PLANES", "MVD_Z_INPLACE", "MVD_PLANE_CAP", "MVD_PLANE_THREADS",
+                          "MVD_ZOCC"})
+      if (std::getenv(v)) return false;
+    return true;
+  }();
+  return on;
+}
+
+namespace {
+
+// A transform length's two radices; r0 == 0: the length has none.
+struct Radices {
+  int r0 = 0, r1 = 0;
+};
+
+constexpr int kPairMaxLen = 400;
+// cost of a plane that leaves one CTA per SM: per voxel of its tiles, 512x512x256 measured 7 to 20%
+// more at 226 KB per plane than at 112 KB
+constexpr double kPairOneCtaCost = 1.1;
+// a plane buffer leaves the epilogues their static shared memory
+constexpr size_t kPairSmemMax = 227 * 1024 - 1024;
+
+// Radix pairs per length, the choice that needs the fewest registers: x stages hold 4 registers
+// per point of either radix, the y stage next to the real step 8 per point of r0 and the other 4
+// per point of r1.
+struct ZRadices {
+  int a = 0, b = 0, c = 0;
+};
+
+struct PairLengths {
+  Radices x[kPairMaxLen + 1], y[kPairMaxLen + 1];
+  ZRadices z[kPairMaxLen + 1];
+  PairLengths() {
+    auto fill = [](Radices* out, std::initializer_list<int> a, std::initializer_list<int> b, int w0) {
+      int best[kPairMaxLen + 1];
+      std::fill(best, best + kPairMaxLen + 1, INT_MAX);
+      for (int r0 : a)
+        for (int r1 : b) {
+          const int n = r0 * r1;
+          if (n > kPairMaxLen) continue;
+          // the larger of the two, then the smaller first radix
+          const int cost = std::max(w0 * r0, r1) * 64 + r0;
+          if (cost < best[n]) {
+            best[n] = cost;
+            out[n] = Radices{r0, r1};
+          }
+        }
+    };
+#define MVD_LIST(R) R,
+    fill(x, {MVD_PAIR_X0(MVD_LIST)}, {MVD_PAIR_X1(MVD_LIST)}, 1);
+    fill(y, {MVD_PAIR_Y0(MVD_LIST)}, {MVD_PAIR_Y1(MVD_LIST)}, 2);
+    // z: two stages where both radices are at most 10, else three; the middle one (c, beside the
+    // kernel spectrum) no larger than the outer one
+    int best[kPairMaxLen + 1];
+    std::fill(best, best + kPairMaxLen + 1, INT_MAX);
+    for (int c : {MVD_PAIR_ZC(MVD_LIST)})
+      for (int a : {MVD_PAIR_Z(MVD_LIST)})
+        for (int b : {MVD_PAIR_Z(MVD_LIST)}) {
+          const int n = a * b * c;
+          if (n > kPairMaxLen || c > a) continue;
+          const int cost = (b > 1 ? 1000 : 0) + 16 * std::max(a, std::max(b, c)) + c;
+          if (cost < best[n]) {
+            best[n] = cost;
+            z[n] = ZRadices{a, b, c};
+          }
+        }
+#undef MVD_LIST
+  }
+};
+
+const PairLengths& pair_lengths() {
+  static const PairLengths l;
+  return l;
+}
+
+struct PairAxis {
+  AxisTiles a;
+  int shift = 0;  // extra halo on the low side (x: even tile origins)
+};
+
+// Tile counts n = 1, 2, ... with the shortest length that covers the axis; x: lengths 2 m.
+template <class Has>
+std::vector<PairAxis> pair_axis_options(int size, int k, Has has, bool x, int off, int nvol) {
+  std::vector<PairAxis> out;
+  int last = -1;
+  for (int n = 1; n <= size && n <= 64; ++n) {
+    const int need = std::max((size + n - 1) / n + k - 1, 2);
+    int T = need;
+    if (x) T += T & 1;
+    while (T <= (x ? 2 : 1) * kPairMaxLen && !has(x ? T / 2 : T)) T += x ? 2 : 1;
+    if (T > (x ? 2 : 1) * kPairMaxLen || T == last) continue;
+    last = T;
+    PairAxis p;
+    p.a.size = size;
+    p.a.k = k;
+    p.a.T = T;
+    p.a.E = T - k + 1;
+    p.a.n = (size + p.a.E - 1) / p.a.E;
+    if (x && nvol % 2 == 0) {
+      // even tile origins (8-byte gathers) where the length has the room for them
+      const int shift = (off - k / 2) & 1;
+      int E = T - k + 1 - shift;
+      if (p.a.n > 1) E -= E & 1;
+      if (E > 0 && (long long)E * p.a.n >= size) {
+        p.a.E = E;
+        p.shift = shift;
+      }
+    }
+    out.push_back(p);
+    if (p.a.E < 8 && p.a.E < size) break;  // smaller tiles would be nearly all halo
+  }
+  return out;
+}
+
+int pair_cols(int m) { return (m + 2) / 2; }  // pairs that hold the m + 1 columns
+int pair_pitch(int m) { return (2 * pair_cols(m)) | 1; }
+// a plane, then the tables: roots of x and y, column units
+size_t pair_plane_smem(int m, int ty) {
+  const int tab = (m + 1) / 2 + (ty + 1) / 2 + m / 2 + 1;
+  return ((size_t)(ty / 2) * pair_pitch(m) + tab) * sizeof(float4);
+}
+
+// CTA size of the plane passes: 128 registers per thread, so 512 threads per SM over the CTAs that
+// fit its shared memory; no more than a stage has work for.
+int pair_plane_threads(const PairShape& s, size_t smem, long long planes) {
+  const int ctas = pair_ctas_per_sm(smem);
+  int t = ctas >= 4 ? 128 : ctas >= 2 ? 256 : 512;
+  if (planes <= 152) t = 512;  // at most one CTA per SM anyway
+  const int work = std::max(std::max(s.ty / 2 * s.r1x, s.ty / 2 * s.r0x), std::max(s.nunits * (s.r1y / 2), s.pc * s.r0y));
+  return std::max(64, std::min(t, (work + 31) / 32 * 32));
+}
+
+// Tile shape and tables for the pair kernels; false when no shape fits (a kernel too large for
+// their lengths).
+bool plan_pairs(ConvPlan& p, int nx, int ny, int nz, int kx, int ky, int kz, const PlanOptions& opt) {
+  const PairLengths& L = pair_lengths();
+  const auto ox = pair_axis_options(nx, kx, [&](int m) { return L.x[m].r0 > 0; }, true, opt.off_x, opt.vol_x > 0 ? opt.vol_x : nx);
+  const auto oy = pair_axis_options(ny, ky, [&](int m) { return L.y[m].r0 > 0; }, false, 0, 0);
+  const auto oz = pair_axis_options(nz, kz, [&](int m) { return L.z[m].a > 0; }, false, 0, 0);
+  const size_t limit = opt.pair_smem ? std::min(opt.pair_smem, kPairSmemMax) : kPairSmemMax;
+  double best = 1e300;
+  const PairAxis *bx = nullptr, *by = nullptr, *bz = nullptr;
+  for (const auto& a : ox)
+    for (const auto& b : oy) {
+      const int m = a.a.T / 2;
+      const size_t smem = pair_plane_smem(m, b.a.T);
+      if (smem > limit) continue;
+      const double ctas = std::min(4, pair_ctas_per_sm(smem));
+      const double plane = 2.0 * pair_cols(m) * b.a.T;
+      for (const auto& c : oz) {
+        const double nt = (double)a.a.n * b.a.n * c.a.n;
+        const double f = ctas >= 2 ? 1.0 : kPairOneCtaCost;
+        // without whole waves the cost is at least this (most shapes end here)
+        if ((4.0 * f + 1.8) * nt * c.a.T * plane / 152.0 >= best) continue;
+        // time of a pass in units of one value of one SM: whole waves of CTAs, those of a wave
+        // sharing the SM
+        auto waves = [](double items, double per_sm, double work) {
+          const double conc = std::min(per_sm, std::ceil(items / 152.0));
+          return std::ceil(items / (152.0 * conc)) * conc * work;
+        };
+        const double cost = (4.0 * f * waves(nt * c.a.T, ctas, plane) +
+                             1.8 * waves(nt * std::ceil(plane / (2.0 * kPairChunk)), 2.0, 2.0 * kPairChunk * c.a.T)) *
+                            (1.0 + 1e-3 * nt);
+        if (cost < best) {
+          best = cost;
+          bx = &a;
+          by = &b;
+          bz = &c;
+        }
+      }
+    }
+  if (!bx) return false;
+  p.ax = bx->a;
+  p.ay = by->a;
+  p.az = bz->a;
+  PairShape& s = p.ps;
+  s.m = p.ax.T / 2;
+  s.ty = p.ay.T;
+  s.tz = p.az.T;
+  s.r0x = L.x[s.m].r0;
+  s.r1x = L.x[s.m].r1;
+  s.r0y = L.y[s.ty].r0;
+  s.r1y = L.y[s.ty].r1;
+  s.az = L.z[s.tz].a;
+  s.bz = L.z[s.tz].b;
+  s.cz = L.z[s.tz].c;
+  s.pc = pair_cols(s.m);
+  s.pitch = pair_pitch(s.m);
+  s.nunits = s.m / 2 + 1;
+  const int plane = s.pc * s.ty;
+  const long long tile_spec = 2LL * plane * s.tz;
+  long long off = 0;
+  for (int iz = 0; iz < p.az.n; ++iz)
+    for (int iy = 0; iy < p.ay.n; ++iy)
+      for (int ix = 0; ix < p.ax.n; ++ix) {
+        TileDesc t{};
+        t.tx = p.ax.T; t.ty = p.ay.T; t.tz = p.az.T;
+        t.px = s.pc;
+        t.pitch = s.pitch;
+        t.hx = kx / 2 + bx->shift; t.hy = ky / 2; t.hz = kz / 2;
+        const int ex0 = ix * p.ax.E, ey0 = iy * p.ay.E, ez0 = iz * p.az.E;
+        t.ox = ex0 - t.hx; t.oy = ey0 - t.hy; t.oz = ez0 - t.hz;
+        t.ex = std::min(p.ax.E, nx - ex0);
+        t.ey = std::min(p.ay.E, ny - ey0);
+        t.ez = std::min(p.az.E, nz - ez0);
+        t.spec_off = off;
+        off += tile_spec;
+        p.tiles.push_back(t);
+      }
+  p.spec_elems = off;
+  p.otf_elems = tile_spec;
+  p.paired = true;
+  p.smem_pair = pair_plane_smem(s.m, s.ty);
+  p.smem_pair_z = ((size_t)s.tz * kPairChunk + (s.tz + 1) / 2 + (s.bz > 1 ? (s.bz * s.cz + 1) / 2 : 0)) * sizeof(float4);
+  p.z_chunks = (plane + kPairChunk - 1) / kPairChunk;
+  p.pair_threads = opt.threads > 0 ? opt.threads : pair_plane_threads(s, p.smem_pair, (long long)p.tiles.size() * s.tz);
+  p.threads_plane = p.pair_threads;
+  return true;
+}
+
+}  // namespace
+
+int pair_ctas_per_sm(size_t smem) {
+  // an SM has 228 KB of shared memory; a CTA takes 1 KB for the system and up to 1 KB statically
+  return (int)std::max<size_t>(1, 228 * 1024 / (smem + 2048));
+}
+
+// The plan's tables in one block: its tiles, the full tile, the stage roots and the column units.
+void ConvPlan::upload_pair() {
+  std::vector<unsigned char> host;
+  auto put = [&](const void* src, size_t bytes) {
+    const size_t at = host.size();
+    host.resize(at + (bytes + 15) / 16 * 16);
+    std::memcpy(host.data() + at, src, bytes);
+    return at;
+  };
+  std::vector<TileDesc> td(tiles);
+  TileDesc full = tiles[0];
+  full.ox = full.oy = full.oz = 0;
+  full.hx = full.hy = full.hz = 0;
+  full.ex = full.tx; full.ey = full.ty; full.ez = full.tz;
+  full.spec_off = 0;
+  td.push_back(full);
+  put(td.data(), td.size() * sizeof(TileDesc));
+  auto root = [](long long num, long long den) {  // exp(-2 pi i num / den)
+    const double a = -2.0 * M_PI * (double)(num % den) / (double)den;
+    return make_float2((float)std::cos(a), (float)std::sin(a));
+  };
+  auto roots = [&](int n, int r0, int r1) {  // W^(j k0) by position r1 k0 + j
+    std::vector<float2> w(n);
+    for (int k0 = 0; k0 < r0; ++k0)
+      for (int j = 0; j < r1; ++j) w[k0 * r1 + j] = root((long long)j * k0, n);
+    return w;
+  };
+  const auto wx = roots(ps.m, ps.r0x, ps.r1x), wy = roots(ps.ty, ps.r0y, ps.r1y), wz = roots(ps.tz, ps.az, ps.bz * ps.cz),
+             wc = roots(ps.bz * ps.cz, ps.bz, ps.cz);
+  // one unit per column pair (f, M - f), f = 0 .. M / 2, ordered by the position of f
+  auto pos = [&](int f) { return (f % ps.r0x) * ps.r1x + f / ps.r0x; };
+  std::vector<PairUnit> un;
+  for (int f = 0; f <= ps.m / 2; ++f) {
+    const float2 w = root(f, 2LL * ps.m);
+    PairUnit u{};
+    u.a = (short)pos(f);
+    u.b_load = (short)(f == 0 ? 0 : pos(ps.m - f));
+    u.b_store = (short)(f == 0 ? ps.m : pos(ps.m - f));
+    u.wx = w.x;
+    u.wy = w.y;
+    un.push_back(u);
+  }
+  std::sort(un.begin(), un.end(), [](const PairUnit& a, const PairUnit& b) { return a.a < b.a; });
+  const size_t ox = put(wx.data(), wx.size() * sizeof(float2)), oy = put(wy.data(), wy.size() * sizeof(float2));
+  const size_t ou = put(un.data(), un.size() * sizeof(PairUnit)), oz = put(wz.data(), wz.size() * sizeof(float2));
+  const size_t oc = ps.bz > 1 ? put(wc.data(), wc.size() * sizeof(float2)) : oz;
+  d_pair.alloc(host.size());
+  upload_table(d_pair.p, host.data(), host.size());
+  const float4* d = d_pair.as<float4>();
+  ps.tab = d + ox / 16;
+  ps.tab_y = (int)((oy - ox) / 16);
+  ps.tab_units = (int)((ou - ox) / 16);
+  ps.ntab = (int)((oz - ox) / 16);
+  ps.tabz = d + oz / 16;
+  ps.ntabz = (int)((host.size() - oz) / 16);
+  ps.tab_c = (int)((oc - oz) / 16);
+  ps.perz = ps.bz > 1 ? ps.bz : ps.az;
+}
+
 std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, int kx, int ky,
                                          int kz, const PlanOptions& opt) {
   if (nx < 1 || ny < 1 || nz < 1) throw std::invalid_argument("empty volume");
   if (kx < 1 || ky < 1 || kz < 1 || !(kx & 1) || !(ky & 1) || !(kz & 1))
     throw std::invalid_argument("kernel sizes must be odd and positive");
+  if (use_pairs() && !opt.scalar) {
+    auto plan = std::make_unique<ConvPlan>();
+    ConvPlan& p = *plan;
+    p.nx = nx; p.ny = ny; p.nz = nz;
+    p.kx = kx; p.ky = ky; p.kz = kz;
+    p.vol[0] = nx; p.vol[1] = ny; p.vol[2] = nz;
+    p.box_hi[0] = nx; p.box_hi[1] = ny; p.box_hi[2] = nz;
+    if (plan_pairs(p, nx, ny, nz, kx, ky, kz, opt)) {
+      p.upload();
+      return plan;
+    }
+  }
   auto opts = [&](int size, int k, bool even, int tmax, int force) {
     if (force > 0) {
       AxisTiles a;
@@ -570,11 +873,11 @@ void build_otf(PlanTable& pt, const ConvPlan& plan, const float* kernel, float2*
       kernel, plan.kx, plan.ky, plan.kz, scratch.as<float>(), tx, ty, tz);
   MVD_CHECK(cudaGetLastError());
   count_launch();
-  // one tile covering the placed kernel volume exactly; its spectrum goes to `otf`
-  launch_fwd_value_items(pt, plan, plan.d_otf_tile.as<TileDesc>(), plan.d_otf_fwd.as<int2>(), plan.n_otf_fwd,
-                         scratch.as<float>(), tx, ty, tz, 0.f, otf, s);
-  launch_z_forward_scaled(pt, plan, plan.d_otf_tile.as<TileDesc>(), plan.d_otf_z.as<int2>(), plan.n_otf_z, otf,
-                          (float)(1.0 / ((double)tx * ty * tz)), s);
+  // one tile covering the placed kernel volume exactly; its spectrum goes to `otf`.  The product of
+  // two spectra carries the passes' scale twice.
+  launch_fwd_value_tiles(pt, plan, TileSet::Full, scratch.as<float>(), tx, ty, tz, 0.f, otf, s);
+  const double sc = spectrum_scale(plan) * spectrum_scale(plan);
+  launch_z_forward(pt, plan, TileSet::Full, otf, (float)(1.0 / (sc * tx * ty * tz)), s);
 }
 
 // ------------------------------------------------------------------------------------------

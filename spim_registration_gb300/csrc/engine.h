@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "kernels.cuh"
+#include "pair_kernels.cuh"
 
 namespace mvd {
 
@@ -114,13 +115,26 @@ struct ConvPlan {
   bool ascending = false;              // radices of every length in ascending order
   bool generic = false;                // run the generic kernels even where a compiled shape exists
   bool staged = false;                 // large compiled planes: in-place kernels, two CTAs per SM
+  // the packed pair kernels (pair_kernels.cuh) run this plan; without them (a tile shape they do
+  // not have, or an option that asks for the scalar kernels) the item tables below are used
+  bool paired = false;
+  PairShape ps{};
+  int pair_threads = 0;                // CTA size of the plane passes
+  int z_chunks = 0;                    // pencil-pair chunks of a tile
+  size_t smem_pair = 0, smem_pair_z = 0;
+  DevBuf d_pair;                       // tiles, one full tile, roots and column units in one block
   DevBuf d_tiles, d_items_fwd, d_items_inv, d_items_z, d_items_zw;
   // one tile of this shape at the origin and its work items: the OTF build's tables
   DevBuf d_otf_tile, d_otf_fwd, d_otf_z;
   int n_otf_fwd = 0, n_otf_z = 0;
   long long padded_voxels() const { return (long long)tiles.size() * ax.T * ay.T * az.T; }
   void upload();
+  void upload_pair();
 };
+
+// The tiles a launch runs over: all of the plan's, or one tile of its shape at the origin whose
+// effective region is the whole tile (kernel spectra, the lags of the PSF gradient).
+enum class TileSet { All, Full };
 
 struct PlanOptions {
   int force_tx = 0, force_ty = 0, force_tz = 0;  // 0 = planner's choice
@@ -128,6 +142,10 @@ struct PlanOptions {
   int threads = 0;                               // plane CTA size; 0 = plane_threads()
   bool ascending = false;                        // radix order of the tile's FFT lengths
   bool generic = false;                          // generic kernels only
+  bool scalar = false;                           // never the packed pair kernels
+  size_t pair_smem = 0;                          // largest plane buffer of a pair plan in bytes (0: no limit)
+  int off_x = 0;                                 // where the covered region will be placed along x,
+  int vol_x = 0;                                 // and the row length there (0: the region is the volume)
 };
 
 // Move a plan's tiles by (dx, dy, dz) into the frame of a larger volume `vol` whose data box
@@ -137,6 +155,13 @@ void place_plan(ConvPlan& p, int dx, int dy, int dz, const int vol[3]);
 // Choose tiles for a (volume, kernel) pair; effective regions cover the whole volume.
 std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, int kx, int ky,
                                          int kz, const PlanOptions& opt = PlanOptions());
+
+// Whether convolutions run the packed pair kernels by default.  MVD_PAIRED=0 selects the scalar
+// kernels, and so does any of the switches that compare those with one another
+// (MVD_FIXED_PLANES, MVD_STAGED_PLANES, MVD_Z_INPLACE, MVD_PLANE_CAP, MVD_PLANE_THREADS, MVD_ZOCC).
+bool use_pairs();
+// CTAs of a pair plan's plane passes an SM holds at once.
+int pair_ctas_per_sm(size_t smem);
 
 // Planner's budget for one plane buffer (complex values).
 int plane_cap();
@@ -202,12 +227,11 @@ inline void set_smem(K kernel, size_t bytes) {
   set_smem_raw(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-// Forward plane pass over explicit tile / item tables, gathering from a (vx, vy, vz) volume
-// with a constant border value; and the forward-only, scaled z pass (OTF preparation).
-void launch_fwd_value_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            const float* vol, int vx, int vy, int vz, float value, float2* spec, cudaStream_t s);
-void launch_z_forward_scaled(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                             float2* spec, float scale, cudaStream_t s);
+// Forward plane pass gathering from a (vx, vy, vz) volume with a constant border value; and the
+// forward-only, scaled z pass (kernel spectra; spectra of the PSF gradient).
+void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float* vol, int vx, int vy, int vz,
+                            float value, float2* spec, cudaStream_t s);
+void launch_z_forward(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, float scale, cudaStream_t s);
 
 // The three passes, for fused use by the deconvolution handle.
 void launch_fwd_mirror(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s);
@@ -226,21 +250,40 @@ long long launch_count();
 void count_launch(int n = 1);
 
 // ---- forward/backward of the Poisson image-formation model (adjoint.cu, passes_*.cu) ----
+// (the PSF gradient's passes take scalar plans only)
 // forward plane pass of `vol` (value 0 outside) keeping only each tile's effective region
 void launch_fwd_masked(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s);
-// forward-only z pass (unscaled) over every tile of p
-void launch_z_forward(PlanTable& pt, const ConvPlan& p, float2* spec, cudaStream_t s);
-// inverse-only z pass over explicit tables
-void launch_z_inverse_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            float2* spec, cudaStream_t s);
-// inverse plane pass storing the effective region of explicit tiles into out (dims nx, ny)
-void launch_inv_store_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            const float2* spec, float* out, int nx, int ny, cudaStream_t s);
+// inverse-only z pass
+void launch_z_inverse(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, cudaStream_t s);
+// inverse plane pass storing the effective region of the tiles into out (dims nx, ny)
+void launch_inv_store_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float2* spec, float* out, int nx,
+                            int ny, cudaStream_t s);
 // inverse plane pass with the NLL epilogue: nll += sum, r = residual (r may be null)
 void launch_inv_nll(PlanTable& pt, const ConvPlan& p, const float2* spec, const float* img, const float* w, float* r,
                     double* nll, cudaStream_t s);
-// acc[i] = sum_t B_t[i] conj(A_t[i]) over `ntiles` tile spectra of `elems` values each
+// acc[i] = sum_t B_t[i] conj(A_t[i]) over `ntiles` tile spectra of `elems` values each (scalar plans)
 void dev_cross_accumulate(const float2* B, const float2* A, int ntiles, long long elems, float2* acc, cudaStream_t s);
+// the factor by which the forward passes of p scale a spectrum (2 for the pair kernels)
+inline double spectrum_scale(const ConvPlan& p) { return p.paired ? 2.0 : 1.0; }
+
+// ---- launches of the pair kernels (pair_fwd.cu, pair_z.cu, pair_inv.cu) ----
+struct PairTiles {
+  const TileDesc* t;
+  int n;
+};
+inline PairTiles pair_tiles(const ConvPlan& p, TileSet set) {
+  const TileDesc* t = p.d_pair.as<TileDesc>();
+  const int n = (int)p.tiles.size();
+  return set == TileSet::All ? PairTiles{t, n} : PairTiles{t + n, 1};
+}
+void pair_fwd_mirror(const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s);
+void pair_fwd_value(const ConvPlan& p, TileSet set, const GatherValue& g, float2* spec, cudaStream_t s);
+void pair_z_conv(const ConvPlan& p, float2* spec, const float2* otf, cudaStream_t s);
+void pair_z_forward(const ConvPlan& p, TileSet set, float2* spec, float scale, cudaStream_t s);  // kernel spectra
+void pair_inv_store(const ConvPlan& p, const float2* spec, const EpiStore& e, cudaStream_t s);
+void pair_inv_quotient(const ConvPlan& p, const float2* spec, const EpiQuotient& e, cudaStream_t s);
+void pair_inv_update(const ConvPlan& p, const float2* spec, const EpiUpdate& e, cudaStream_t s);
+void pair_inv_nll(const ConvPlan& p, const float2* spec, const EpiNll& e, cudaStream_t s);
 // G[j] = scale * R[(j - k/2) mod T] for the kernel-sized output G (circular lags of a tile)
 void dev_extract_lags(const float* R, int tx, int ty, int tz, int kx, int ky, int kz, float scale, float* G,
                       cudaStream_t s);

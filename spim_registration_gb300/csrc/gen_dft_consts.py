@@ -1,6 +1,7 @@
 """Writes dft_consts.cuh: exp(-2 pi i m / R) for the composite register DFT sizes.
 
-The values are the roots of unity computed here in double precision and rounded to float.
+The values are the roots of unity computed here in double precision and rounded to float: as
+``wconst`` in constant memory, and as ``wroot`` in literals (for the packed DFTs of pair_fft.cuh).
 Run:  python spim_registration_gb300/csrc/gen_dft_consts.py
 """
 import math
@@ -18,6 +19,17 @@ for r in SIZES:
 out += ["", "template <int R>", "__device__ __forceinline__ float2 wconst(int m);"]
 for r in SIZES:
     out.append(f"template <> __device__ __forceinline__ float2 wconst<{r}>(int m) {{ return c_w{r}[m]; }}")
+# the same roots as literals (a constant index after unrolling folds to an immediate), zeros exact
+out += ["", "template <int R>", "__device__ __forceinline__ float2 wroot(int m);"]
+for r in SIZES:
+    vals = []
+    for m in range(r):
+        a = -2.0 * math.pi * m / r
+        x, y = [0.0 if abs(v) < 1e-12 else v for v in (math.cos(a), math.sin(a))]
+        vals.append("{%.9ef, %.9ef}" % (x, y))
+    out.append(f"template <> __device__ __forceinline__ float2 wroot<{r}>(int m) {{")
+    out.append(f"  const float2 t[{r}] = {{" + ", ".join(vals) + "};")
+    out += ["  return t[m];", "}"]
 out += ["", "}  // namespace mvd", ""]
 path = os.path.join(os.path.dirname(os.path.abspath(__file__)), "dft_consts.cuh")
 open(path, "w").write("\n".join(out))

@@ -181,6 +181,13 @@ struct EpiStore {
   int nx, ny;
   int inputs(const float** p) const { return 0; }  // volumes the epilogue reads (for L2 prefetch)
   __device__ __forceinline__ void acc_init() {}
+  // for callers that do the loads and stores themselves: the input volumes (kIn of them), the
+  // output volume (null: none) and the result of one voxel
+  static constexpr int kIn = 0;
+  __device__ __forceinline__ const float* src0() const { return nullptr; }
+  __device__ __forceinline__ const float* src1() const { return nullptr; }
+  __device__ __forceinline__ float* dst() const { return out; }
+  __device__ __forceinline__ float value(float v, float, float) { return v; }
   __device__ __forceinline__ void operator()(long long g, float v) { out[g] = v; }
   template <int K>
   __device__ __forceinline__ void apply(long long g0, const int* off, const float* val, const bool* ok) {
@@ -204,6 +211,11 @@ struct EpiQuotient {
   __device__ __forceinline__ static float quotient(float i, float blurred) {
     return i > 0.f ? __fdividef(i, blurred) : 1.f;  // within 2 ulp (blurred below 2^126)
   }
+  static constexpr int kIn = 1;
+  __device__ __forceinline__ const float* src0() const { return img; }
+  __device__ __forceinline__ const float* src1() const { return nullptr; }
+  __device__ __forceinline__ float* dst() const { return q; }
+  __device__ __forceinline__ float value(float blurred, float i, float) { return quotient(i, blurred); }
   __device__ __forceinline__ void operator()(long long g, float blurred) { q[g] = quotient(__ldg(img + g), blurred); }
   template <int K>
   __device__ __forceinline__ void apply(long long g0, const int* off, const float* val, const bool* ok) {
@@ -262,25 +274,30 @@ struct EpiUpdate {
   }
   __device__ __forceinline__ float next_value(float last, float integral, float w) {
     const float value = __fmul_rn(last, integral);
-    float adjusted;
-    if (value > 0.f) {
-      if (lambda > 0.f && !isinf(value)) {
-        const float x = __fadd_rn(1.f, __fmul_rn(2.f * lambda, value));
-        const float r = __fmul_rn(x, rsqrtf(x));
-        adjusted = __fdividef(__fmul_rn(2.f, value), __fadd_rn(r, 1.f));
-      } else {
-        adjusted = value;
-      }
-    } else {
-      adjusted = 1e-4f;
+    // value <= 0 and NaN give something that is not above minValue, or NaN: both become minValue in
+    // the maximum (fmaxf returns its other operand for a NaN)
+    float adjusted = value;
+    if (lambda > 0.f) {
+      const float x = __fadd_rn(1.f, __fmul_rn(2.f * lambda, value));
+      float rs, inv;
+      asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rs) : "f"(x));  // x >= 1 wherever the value counts
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(__fadd_rn(__fmul_rn(x, rs), 1.f)));
+      adjusted = __fmul_rn(__fmul_rn(2.f, value), inv);
+      adjusted = isinf(value) ? value : adjusted;
     }
-    const float next = isnan(adjusted) ? 1e-4f : fmaxf(1e-4f, adjusted);
+    const float next = fmaxf(1e-4f, adjusted);
     const float out = __fadd_rn(last, __fmul_rn(__fsub_rn(next, last), w));
     const float change = fabsf(__fsub_rn(out, last));
     acc_sum += change;
     acc_max = fmaxf(acc_max, change);
     return out;
   }
+  static constexpr int kIn = 2;
+  __device__ __forceinline__ const float* src0() const { return psi; }
+  __device__ __forceinline__ const float* src1() const { return weight; }
+  __device__ __forceinline__ float* dst() const { return psi; }
+  // (0, 0) inputs change nothing and add nothing to the statistics, whatever the integral
+  __device__ __forceinline__ float value(float integral, float last, float w) { return next_value(last, integral, w); }
   __device__ __forceinline__ void operator()(long long g, float integral) {
     psi[g] = next_value(psi[g], integral, __ldg(weight + g));
   }
@@ -374,6 +391,15 @@ struct EpiNll {
     }
     res = 0.f;
     return 0.f;
+  }
+  static constexpr int kIn = 2;
+  __device__ __forceinline__ const float* src0() const { return img; }
+  __device__ __forceinline__ const float* src1() const { return weight; }
+  __device__ __forceinline__ float* dst() const { return r; }
+  __device__ __forceinline__ float value(float f, float im, float w) {
+    float res;
+    acc += term(f, im, w, res);
+    return res;
   }
   __device__ __forceinline__ void operator()(long long g, float f) {
     float res;

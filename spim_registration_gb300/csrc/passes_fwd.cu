@@ -128,6 +128,7 @@ static void launch_fwd_impl(PlanTable& pt, const TileDesc* tiles, const int2* it
 }
 
 void launch_fwd_mirror(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s) {
+  if (p.paired) return pair_fwd_mirror(p, vol, spec, s);
   GatherMirror g{{vol, p.vol[0], p.vol[1], p.vol[2]}};
   launch_fwd_impl(pt, p.d_tiles.as<TileDesc>(), p.d_items_fwd.as<int2>(), (int)p.items_fwd.size(), p.smem_plane,
                   p.threads_plane, p.ax.T, p.ay.T, spec, g, s, p.generic, p.staged);
@@ -137,14 +138,19 @@ void launch_fwd_value(PlanTable& pt, const ConvPlan& p, const float* vol, float 
                       cudaStream_t s) {
   GatherValue g = GatherValue::box(vol, p.vol[0], p.vol[1], p.vol[2], value, p.box_lo[0], p.box_lo[1], p.box_lo[2],
                                    p.box_hi[0], p.box_hi[1], p.box_hi[2]);
+  if (p.paired) return pair_fwd_value(p, TileSet::All, g, spec, s);
   launch_fwd_impl(pt, p.d_tiles.as<TileDesc>(), p.d_items_fwd.as<int2>(), (int)p.items_fwd.size(), p.smem_plane,
                   p.threads_plane, p.ax.T, p.ay.T, spec, g, s, p.generic, p.staged);
 }
 
-void launch_fwd_value_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            const float* vol, int vx, int vy, int vz, float value, float2* spec, cudaStream_t s) {
+void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float* vol, int vx, int vy, int vz,
+                            float value, float2* spec, cudaStream_t s) {
   GatherValue g = GatherValue::full(vol, vx, vy, vz, value);
-  launch_fwd_impl(pt, tiles, items, nitems, p.smem_plane, p.threads_plane, p.ax.T, p.ay.T, spec, g, s, p.generic);
+  if (p.paired) return pair_fwd_value(p, set, g, spec, s);
+  const bool all = set == TileSet::All;
+  launch_fwd_impl(pt, (all ? p.d_tiles : p.d_otf_tile).as<TileDesc>(), (all ? p.d_items_fwd : p.d_otf_fwd).as<int2>(),
+                  all ? (int)p.items_fwd.size() : p.n_otf_fwd, p.smem_plane, p.threads_plane, p.ax.T, p.ay.T, spec, g,
+                  s, p.generic);
 }
 
 void launch_fwd_masked(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s) {

@@ -72,12 +72,14 @@ static void launch_inv_impl(PlanTable& pt, const ConvPlan& p, const float2* spec
 
 void launch_inv_store(PlanTable& pt, const ConvPlan& p, const float2* spec, float* out, cudaStream_t s) {
   EpiStore e{out, p.vol[0], p.vol[1]};
+  if (p.paired) return pair_inv_store(p, spec, e, s);
   launch_inv_impl(pt, p, spec, e, s);
 }
 
 void launch_inv_quotient(PlanTable& pt, const ConvPlan& p, const float2* spec, const float* img, float* q,
                          cudaStream_t s) {
   EpiQuotient e{img, q, p.vol[0], p.vol[1]};
+  if (p.paired) return pair_inv_quotient(p, spec, e, s);
   launch_inv_impl(pt, p, spec, e, s);
 }
 
@@ -85,17 +87,24 @@ void launch_inv_update(PlanTable& pt, const ConvPlan& p, const float2* spec, flo
                        float lambda, double* stat_sum, unsigned* stat_max, const StatArchive& archive,
                        cudaStream_t s) {
   EpiUpdate e{psi, weight, lambda, stat_sum, stat_max, p.vol[0], p.vol[1], 0.f, 0.f, archive};
+  if (p.paired) return pair_inv_update(p, spec, e, s);
   launch_inv_impl(pt, p, spec, e, s);
 }
 
 void launch_inv_nll(PlanTable& pt, const ConvPlan& p, const float2* spec, const float* img, const float* w, float* r,
                     double* nll, cudaStream_t s) {
   EpiNll e{img, w, r, nll, p.vol[0], p.vol[1], 0.f};
+  if (p.paired) return pair_inv_nll(p, spec, e, s);
   launch_inv_impl(pt, p, spec, e, s);
 }
 
-void launch_inv_store_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            const float2* spec, float* out, int nx, int ny, cudaStream_t s) {
+void launch_inv_store_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float2* spec, float* out, int nx,
+                            int ny, cudaStream_t s) {
+  if (p.paired) return pair_inv_store(p, spec, EpiStore{out, nx, ny}, s);  // TileSet::All
+  const bool all = set == TileSet::All;
+  const TileDesc* tiles = (all ? p.d_tiles : p.d_otf_tile).as<TileDesc>();
+  const int2* items = (all ? p.d_items_inv : p.d_otf_fwd).as<int2>();  // the full tile: every slice
+  const int nitems = all ? (int)p.items_inv.size() : p.n_otf_fwd;
   if (nitems == 0) return;
   if (!launch_inv_fixed(pt, p, tiles, items, nitems, spec, EpiStore{out, nx, ny}, s)) {
     auto k = plane_inv_kernel<EpiStore>;

@@ -156,6 +156,7 @@ int tensor_dft_failures() {
 }
 
 void launch_z(PlanTable& pt, const ConvPlan& p, float2* spec, const float2* otf, cudaStream_t s) {
+  if (p.paired) return pair_z_conv(p, spec, otf, s);
   if (p.items_z.empty()) return;
   if (p.tensor_dft && !p.generic && launch_z_tc(pt, p, spec, otf, s)) {
     MVD_CHECK(cudaGetLastError());
@@ -175,26 +176,27 @@ void launch_z(PlanTable& pt, const ConvPlan& p, float2* spec, const float2* otf,
   count_launch();
 }
 
-void launch_z_forward_scaled(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                             float2* spec, float scale, cudaStream_t s) {
+void launch_z_forward(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, float scale, cudaStream_t s) {
+  if (p.paired) return pair_z_forward(p, set, spec, scale, s);
+  const bool all = set == TileSet::All;
+  const int nitems = all ? (int)p.items_z.size() : p.n_otf_z;
   if (nitems == 0) return;
   auto k = zpass_kernel<1>;
   set_smem(k, p.smem_z);
-  k<<<nitems, kZThreads, p.smem_z, s>>>(tiles, items, pt.device(), spec, nullptr, scale);
+  k<<<nitems, kZThreads, p.smem_z, s>>>((all ? p.d_tiles : p.d_otf_tile).as<TileDesc>(),
+                                        (all ? p.d_items_z : p.d_otf_z).as<int2>(), pt.device(), spec, nullptr, scale);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }
 
-void launch_z_forward(PlanTable& pt, const ConvPlan& p, float2* spec, cudaStream_t s) {
-  launch_z_forward_scaled(pt, p, p.d_tiles.as<TileDesc>(), p.d_items_z.as<int2>(), (int)p.items_z.size(), spec, 1.f, s);
-}
-
-void launch_z_inverse_items(PlanTable& pt, const ConvPlan& p, const TileDesc* tiles, const int2* items, int nitems,
-                            float2* spec, cudaStream_t s) {
+void launch_z_inverse(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, cudaStream_t s) {
+  const bool all = set == TileSet::All;
+  const int nitems = all ? (int)p.items_z.size() : p.n_otf_z;
   if (nitems == 0) return;
   auto k = zpass_kernel<2>;
   set_smem(k, p.smem_z);
-  k<<<nitems, kZThreads, p.smem_z, s>>>(tiles, items, pt.device(), spec, nullptr, 1.f);
+  k<<<nitems, kZThreads, p.smem_z, s>>>((all ? p.d_tiles : p.d_otf_tile).as<TileDesc>(),
+                                        (all ? p.d_items_z : p.d_otf_z).as<int2>(), pt.device(), spec, nullptr, 1.f);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -300,7 +300,7 @@ class Deconvolution:
         th, var = ctypes.c_int(), ctypes.c_int()
         native.check(self.lib.mvd_get_plan_variant(self.h, view, ctypes.byref(th), ctypes.byref(var)))
         return dict(tiles=tuple(t), tile=tuple(s), effective=tuple(e), padded_voxels=pv.value,
-                    threads=th.value, kernels="compiled" if var.value & 1 else "generic",
+                    threads=th.value, kernels="paired" if var.value & 16 else "compiled" if var.value & 1 else "generic",
                     radix_order="ascending" if var.value & 2 else "descending",
                     tensor_dft=bool(var.value & 4), staged=bool(var.value & 8))
 
