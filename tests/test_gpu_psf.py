@@ -74,3 +74,16 @@ def test_extract_psf_class_per_view_and_average():
     avg = ex.computeAverageTransformedPSF()
     assert avg.shape == tuple(ex.computeMaxDimTransformedPSF()[::-1])
     assert avg.sum() == pytest.approx(sum(p.sum() for p in ex.getPSFMap().values()), rel=1e-5)
+
+
+@pytest.mark.parametrize("shape,psf,beads", [((5, 6, 7), (9, 11, 13), 3),      # PSF larger than the view
+                                             ((20, 30, 70), (33, 5, 9), 40),   # partial runs along x, y and z
+                                             ((16, 16, 16), (1, 1, 1), 200), ((24, 40, 40), (31, 31, 61), 1)])
+def test_extraction_runs_and_bead_chunks_match_oracle(shape, psf, beads):
+    """Runs of 4 x 8 voxels and 32 lanes that end inside the PSF, bead counts around the chunk size,
+    locations outside the view on both sides (periodic) and on voxel centres."""
+    rng = np.random.default_rng(beads)
+    img = (rng.random(shape) * 100).astype(np.float32)
+    locs = rng.uniform(-2, 3, (beads, 3)) * np.array(shape[::-1])
+    locs[0] = np.round(locs[0])
+    _close(extract_psf_local(img, locs, psf), O.extract_psf_local(img, locs, psf))
