@@ -10,15 +10,22 @@
 // out[x] = sum_{j=-R..R} in[x + j] k[R - j] (R = K / 2), accumulated in float in order of j.
 //
 // GPU layout: one pass per axis, out of place between two device buffers.
-//  * x pass: a CTA loads a row segment and its halo into shared memory (coalesced), each
-//    thread computes PX consecutive outputs from a sliding register window.
-//  * y / z pass: a CTA loads a 32-wide (x) slab of CH axis positions plus the halo into shared
-//    memory (each warp reads 32 consecutive floats of one axis position), each thread computes
-//    PA consecutive outputs along the axis for its x.
+//  * x pass, K <= 31 (and 63 for some widths): a warp takes 128 (or 64) x positions of a run of rows.
+//    It keeps the row with its halo in its own shared rows, the following rows already in registers,
+//    and each lane computes 4 (2) consecutive outputs from aligned 16-byte (8-byte) units of the row,
+//    which are neighbours in shared memory from lane to lane (no bank conflicts).
+//  * y / z pass, K <= 31: a thread walks along the axis with the 2R + 1 partial sums of the outputs it
+//    passes in registers: s[m] = in * t[m] + s[m - 1] shifts them by one position and adds the new
+//    value to each, and s[2R] is complete.  No shared memory, every input read once, and the order of
+//    additions stays that of a direct sum.  320x288x190, K = 15: 24.7 us a pass (5.7 TB/s), against 53
+//    us through shared-memory slabs; 31 taps 35 against 66 us.
+//  * y / z pass, K = 63, 127 (bound by arithmetic): a CTA loads a 32-wide (x) slab of CH axis positions
+//    plus the halo into shared memory, each thread computes PA consecutive outputs along the axis.
 // Taps travel as kernel parameters (uniform reads from the constant bank).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <memory>
@@ -53,11 +60,87 @@ __device__ __forceinline__ float fetch(const float* __restrict__ p, long long ba
 }
 
 // ---- x pass --------------------------------------------------------------------------------
-constexpr int kPX = 4;       // outputs per thread
 constexpr int kXThreads = 128;
 
+// P outputs per lane (32 P x positions per warp), `run` rows per warp
+template <int R, int P>
+__global__ void __launch_bounds__(kXThreads, R <= 7 ? 6 : R <= 15 ? 4 : 3) sep_x_kernel(const float* __restrict__ in, float* __restrict__ out, int w,
+                                                          long long rows, int run, Taps taps, int oob, float value) {
+  constexpr int HALO = (R + P - 1) / P * P;  // so that a lane's window starts at a multiple of P
+  constexpr int PER = (32 * P + 2 * HALO + 31) / 32, kAhead = 4;
+  __shared__ __align__(16) float shared[kXThreads / 32][2][PER * 32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int xt = (w + 32 * P - 1) / (32 * P);
+  const long long item = (long long)blockIdx.x * (kXThreads / 32) + warp;
+  const long long r0 = item / xt * run, r1 = min(rows, r0 + run);
+  if (r0 >= rows) return;
+  const int xb = (int)(item % xt) * 32 * P, x = xb + P * lane;
+  const float outside = oob == OOB_VALUE ? value : 0.f;
+  int col[PER];  // this lane's elements of a row: x positions, -1 outside (extended: the border's)
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int c = xb - HALO + lane + 32 * k;
+    col[k] = oob == OOB_EXTEND ? min(max(c, 0), w - 1) : (c >= 0 && c < w ? c : -1);
+  }
+  auto load = [&](float* v, long long r) {
+    if (r >= r1) return;
+    const float* p = in + r * w;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) v[k] = col[k] >= 0 ? __ldg(p + col[k]) : outside;
+  };
+  float ahead[kAhead][PER] = {};
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k) load(ahead[k], r0 + k);
+  const bool vec = (w % P) == 0 && (reinterpret_cast<uintptr_t>(out) & (4 * P - 1)) == 0;
+  for (long long rb = r0; rb < r1; rb += kAhead) {
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) {
+      const long long r = rb + k;
+      if (r >= r1) break;
+      float* s = shared[warp][k & 1];  // the other row's readers are past the barrier between
+#pragma unroll
+      for (int e = 0; e < PER; ++e) s[lane + 32 * e] = ahead[k][e];
+      __syncwarp();
+      load(ahead[k], r + kAhead);
+      float acc[P];
+#pragma unroll
+      for (int o = 0; o < P; ++o) acc[o] = 0.f;
+#pragma unroll
+      for (int e = 0; e < (P + 2 * HALO) / P; ++e) {
+        float v[P];
+        if (P == 4)
+          *reinterpret_cast<float4*>(v) = reinterpret_cast<const float4*>(s)[lane + e];
+        else
+          *reinterpret_cast<float2*>(v) = reinterpret_cast<const float2*>(s)[lane + e];
+#pragma unroll
+        for (int c = 0; c < P; ++c)
+#pragma unroll
+          for (int o = 0; o < P; ++o) {
+            const int m = P * e + c - o - (HALO - R);
+            if (m >= 0 && m <= 2 * R) acc[o] = __fmaf_rn(v[c], taps.k[m >= 0 && m <= 2 * R ? m : 0], acc[o]);
+          }
+      }
+      float* d = out + r * w + x;
+      if (vec && x < w) {
+        if (P == 4)
+          *reinterpret_cast<float4*>(d) = *reinterpret_cast<const float4*>(acc);
+        else
+          *reinterpret_cast<float2*>(d) = *reinterpret_cast<const float2*>(acc);
+      } else {
+#pragma unroll
+        for (int o = 0; o < P; ++o)
+          if (x + o < w) d[o] = acc[o];
+      }
+    }
+  }
+}
+
+// K = 63, 127: a CTA loads 512 outputs' worth of a row and its halo into shared memory, each thread
+// computes 4 consecutive outputs from a sliding register window
+constexpr int kPX = 4;       // outputs per thread
+
 template <int R>
-__global__ void __launch_bounds__(kXThreads) sep_x_kernel(const float* __restrict__ in, float* __restrict__ out,
+__global__ void __launch_bounds__(kXThreads) sep_x_wide_kernel(const float* __restrict__ in, float* __restrict__ out,
                                                           int w, long long rows, Taps taps, int oob, float value) {
   constexpr int SEG = kXThreads * kPX;
   __shared__ float s[SEG + 2 * R + 1];
@@ -134,28 +217,170 @@ __global__ void __launch_bounds__(32 * kAWarps) sep_axis_kernel(const float* __r
     if (a0 + al + q < n) out[base + (long long)(a0 + al + q) * sa] = acc[q];
 }
 
-// The sliding window loads one element past the last tap (win[P-1] after the last FMA), so
-// the shared buffers carry one extra slot: x holds SEG + 2R + 1 elements (the last thread
-// reads up to index SEG - PX + PX + 2R), the axis slab CH + 2R + 1 rows.
+// The sliding window loads one element past the last tap (win[P-1] after the last FMA), so the slab
+// carries one extra row: CH + 2R + 1.
+
+// ---- walks (K <= 31) -----------------------------------------------------------------------
+constexpr int kWalkThreads = 128;
+
+// one step of the partial sums: v becomes tap m of the output that had taps 0 .. m - 1
+template <int R>
+__device__ __forceinline__ float walk_step(float* s, float v, const Taps& t) {
+#pragma unroll
+  for (int m = 2 * R; m > 0; --m) s[m] = __fmaf_rn(v, t.k[m], s[m - 1]);
+  s[0] = __fmaf_rn(v, t.k[0], 0.f);
+  return s[2 * R];
+}
+
+// Along one axis of length n (stride sa): thread p of the other two axes' positions (x + w o at
+// x + o so), outputs [a0, a0 + seg) of the axis.  kAhead inputs are loaded ahead of their use.
+template <int R>
+__global__ void __launch_bounds__(kWalkThreads) sep_walk_kernel(const float* __restrict__ in, float* __restrict__ out,
+                                                                int w, long long positions, int n, long long sa,
+                                                                long long so, int seg, Taps taps, int oob, float value) {
+  constexpr int kAhead = 12;
+  const long long p = (long long)blockIdx.x * kWalkThreads + threadIdx.x;
+  if (p >= positions) return;
+  const long long base = so == w ? p : p / w * so + p % w;
+  const int a0 = blockIdx.y * seg, a1 = min(n, a0 + seg);
+  const float outside = oob == OOB_VALUE ? value : 0.f;
+  const float* src = in + base;
+  float* dst = out + base;
+  float s[2 * R + 1];
+#pragma unroll
+  for (int m = 0; m <= 2 * R; ++m) s[m] = 0.f;
+  auto fetch1 = [&](int i) {
+    if (i >= 0 && i < n) return __ldg(src + (long long)i * sa);
+    return oob == OOB_EXTEND ? __ldg(src + (long long)(i < 0 ? 0 : n - 1) * sa) : outside;
+  };
+  auto fetch = [&](float* v, int i0) {  // inputs i0 .. i0 + kAhead - 1 (those the segment needs)
+    if (i0 >= 0 && i0 + kAhead <= n) {
+      const float* q = src + (long long)i0 * sa;
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) v[k] = __ldg(q + k * sa);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) v[k] = i0 + k < a1 + R ? fetch1(i0 + k) : 0.f;
+    }
+  };
+  float v[kAhead];
+  fetch(v, a0 - R);
+  for (int i0 = a0 - R; i0 < a1 + R; i0 += kAhead) {
+    float next[kAhead];
+    if (i0 + kAhead < a1 + R) fetch(next, i0 + kAhead);
+    const int o0 = i0 - R;
+    float* d = dst + (long long)o0 * sa;
+    if (o0 >= a0 && o0 + kAhead <= a1) {
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) d[k * sa] = walk_step<R>(s, v[k], taps);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kAhead; ++k) {
+        const float r = walk_step<R>(s, v[k], taps);
+        if (o0 + k >= a0 && o0 + k < a1) d[k * sa] = r;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < kAhead; ++k) v[k] = next[k];
+  }
+}
+
+// Outputs per segment of an axis of length n: whole waves of warps (`resident` at once on the GPU),
+// each walking 2 R positions before its first output; the segment count that walks least in all.
+int walk_segment(int n, long long warps_per_segment, long long resident, int R) {
+  int best = n;
+  double cost = 1e300;
+  for (int segs = 1; segs <= n && segs <= 64; ++segs) {
+    const int seg = (n + segs - 1) / segs;
+    const double waves = std::ceil((double)warps_per_segment * segs / resident);
+    const double c = waves * (seg + 2 * R + 4);
+    if (c < cost) {
+      cost = c;
+      best = seg;
+    }
+  }
+  return best;
+}
+
+// warps of a kernel resident at once on the current device (kWalkThreads per block)
+template <class K>
+long long resident_warps(K kernel) {
+  int dev = 0, sms = 0, blocks = 0;
+  MVD_CHECK(cudaGetDevice(&dev));
+  MVD_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  MVD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kWalkThreads, 0));
+  return (long long)sms * std::max(1, blocks) * (kWalkThreads / 32);
+}
 
 template <int R>
-void launch_pass(int axis, const float* in, float* out, int w, int h, int d, const Taps& t, int oob, float value,
+void launch_walk(int axis, const float* in, float* out, int w, int h, int d, const Taps& t, int oob, float value,
                  cudaStream_t s) {
-  if (axis == 0) {
-    const long long rows = (long long)h * d;
-    const int gx = (w + kXThreads * kPX - 1) / (kXThreads * kPX);
-    const long long gy = std::min<long long>(rows, 65535);
-    const long long gz = (rows + gy - 1) / gy;
-    sep_x_kernel<R><<<dim3(gx, (unsigned)gy, (unsigned)gz), kXThreads, 0, s>>>(in, out, w, rows, t, oob, value);
-  } else {
-    const int n = axis == 1 ? h : d;
-    const long long sa = axis == 1 ? (long long)w : (long long)w * h;
-    const long long so = axis == 1 ? (long long)w * h : (long long)w;
-    const int outer = axis == 1 ? d : h;
-    if (outer > 65535 || (n + kCH - 1) / kCH > 65535) throw std::invalid_argument("image too large for the y/z passes");
-    sep_axis_kernel<R><<<dim3((w + 31) / 32, (n + kCH - 1) / kCH, outer), 32 * kAWarps, 0, s>>>(in, out, w, n, sa, so,
-                                                                                             t, oob, value);
+  const int n = axis == 1 ? h : d;
+  const long long sa = axis == 1 ? (long long)w : (long long)w * h;
+  const long long so = axis == 1 ? (long long)w * h : (long long)w;
+  const int outer = axis == 1 ? d : h;
+  if (outer > 65535 || (n + kCH - 1) / kCH > 65535) throw std::invalid_argument("image too large for the y/z passes");
+  const long long positions = (long long)w * outer;
+  const long long blocks = (positions + kWalkThreads - 1) / kWalkThreads;
+  int seg = walk_segment(n, blocks * (kWalkThreads / 32), resident_warps(sep_walk_kernel<R>), R);
+  seg = std::max(seg, (n + 65534) / 65535);
+  sep_walk_kernel<R><<<dim3((unsigned)blocks, (n + seg - 1) / seg), kWalkThreads, 0, s>>>(in, out, w, positions, n, sa, so,
+                                                                                       seg, t, oob, value);
+  MVD_CHECK(cudaGetLastError());
+  count_launch();
+}
+
+template <int R, int P>
+void launch_x_of(const float* in, float* out, int w, long long rows, const Taps& t, int oob, float value, cudaStream_t s) {
+  const int xt = (w + 32 * P - 1) / (32 * P);
+  // two waves of warps; at most 64 rows each
+  const long long warps = 2 * resident_warps(sep_x_kernel<R, P>);
+  const int run = (int)std::max(1LL, std::min(64LL, rows * xt / warps));
+  const long long blocks = ((rows + run - 1) / run * xt + kXThreads / 32 - 1) / (kXThreads / 32);
+  if (blocks > 0x7fffffffLL) throw std::invalid_argument("image too large for the x pass");
+  sep_x_kernel<R, P><<<(unsigned)blocks, kXThreads, 0, s>>>(in, out, w, rows, run, t, oob, value);
+  MVD_CHECK(cudaGetLastError());
+  count_launch();
+}
+
+// Which x kernel: measured on 320x288x190 / 512x256x128 / 200x300x250 (us, row runs against 512-wide
+// segments): K = 15 39.6 / 36.2 / 38.8 against 56.1 / 41.4 / 91.8; K = 31 58.6 / 44.9 / 52.3 against
+// 66.3 / 49.3 / 102; K = 63 89.2 / 79.3 / 91.8 against 90.2 / 70.1 / 125; K = 127 174 / 192 / 227
+// against 141 / 122 / 173.  So up to 31 taps take the row runs; 63 take them where more than 0.4 of
+// the segments' outputs lie past the row's end; 127 (a 132-value window per lane) never do.
+template <int R>
+void launch_x(const float* in, float* out, int w, int h, int d, const Taps& t, int oob, float value, cudaStream_t s) {
+  const long long rows = (long long)h * d;
+  const int gx = (w + kXThreads * kPX - 1) / (kXThreads * kPX);
+  if constexpr (R >= 31) {
+    if (R > 31 || 10LL * w >= 6LL * gx * kXThreads * kPX) {
+      const long long gy = std::min<long long>(rows, 65535);
+      const long long gz = (rows + gy - 1) / gy;
+      sep_x_wide_kernel<R><<<dim3(gx, (unsigned)gy, (unsigned)gz), kXThreads, 0, s>>>(in, out, w, rows, t, oob, value);
+      MVD_CHECK(cudaGetLastError());
+      count_launch();
+      return;
+    }
   }
+  if constexpr (R <= 31) {
+    // 4 outputs per lane unless 64-wide tiles leave fewer lanes idle at the end of a row
+    if ((w + 63) / 64 * 64 < (w + 127) / 128 * 128)
+      launch_x_of<R, 2>(in, out, w, rows, t, oob, value, s);
+    else
+      launch_x_of<R, 4>(in, out, w, rows, t, oob, value, s);
+  }
+}
+
+template <int R>
+void launch_axis(int axis, const float* in, float* out, int w, int h, int d, const Taps& t, int oob, float value,
+                 cudaStream_t s) {
+  const int n = axis == 1 ? h : d;
+  const long long sa = axis == 1 ? (long long)w : (long long)w * h;
+  const long long so = axis == 1 ? (long long)w * h : (long long)w;
+  const int outer = axis == 1 ? d : h;
+  if (outer > 65535 || (n + kCH - 1) / kCH > 65535) throw std::invalid_argument("image too large for the y/z passes");
+  sep_axis_kernel<R><<<dim3((w + 31) / 32, (n + kCH - 1) / kCH, outer), 32 * kAWarps, 0, s>>>(in, out, w, n, sa, so, t,
+                                                                                           oob, value);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }
@@ -163,11 +388,11 @@ void launch_pass(int axis, const float* in, float* out, int w, int h, int d, con
 void run_pass(int taps_len, int axis, const float* in, float* out, int w, int h, int d, const Taps& t, int oob,
               float value, cudaStream_t s) {
   switch (taps_len) {
-    case 7: launch_pass<3>(axis, in, out, w, h, d, t, oob, value, s); break;
-    case 15: launch_pass<7>(axis, in, out, w, h, d, t, oob, value, s); break;
-    case 31: launch_pass<15>(axis, in, out, w, h, d, t, oob, value, s); break;
-    case 63: launch_pass<31>(axis, in, out, w, h, d, t, oob, value, s); break;
-    case 127: launch_pass<63>(axis, in, out, w, h, d, t, oob, value, s); break;
+    case 7: return axis ? launch_walk<3>(axis, in, out, w, h, d, t, oob, value, s) : launch_x<3>(in, out, w, h, d, t, oob, value, s);
+    case 15: return axis ? launch_walk<7>(axis, in, out, w, h, d, t, oob, value, s) : launch_x<7>(in, out, w, h, d, t, oob, value, s);
+    case 31: return axis ? launch_walk<15>(axis, in, out, w, h, d, t, oob, value, s) : launch_x<15>(in, out, w, h, d, t, oob, value, s);
+    case 63: return axis ? launch_axis<31>(axis, in, out, w, h, d, t, oob, value, s) : launch_x<31>(in, out, w, h, d, t, oob, value, s);
+    case 127: return axis ? launch_axis<63>(axis, in, out, w, h, d, t, oob, value, s) : launch_x<63>(in, out, w, h, d, t, oob, value, s);
     default: throw std::invalid_argument("unsupported kernel size");
   }
 }

@@ -116,3 +116,25 @@ def test_invalid_arguments_leave_the_image_unchanged():
                                    1, 2, 0.0, 0)  # x requested without its kernel
     np.testing.assert_array_equal(img, 1.0)
     assert OutOfBounds.EXTEND_BORDER_PIXELS == 2
+
+
+@pytest.mark.parametrize("K", [7, 15, 31, 63, 127])
+@pytest.mark.parametrize("oob", [0, 1, 2])
+@pytest.mark.parametrize("shape", [(37, 230, 171), (3, 198, 200), (70, 40, 320)])
+def test_rows_and_walks_match_oracle(K, oob, shape):
+    """Row runs and walk segments that end inside the image, widths that are and are not multiples of
+    2 and 4 (128- and 64-wide row tiles), and axes shorter than the kernel."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(K + oob + shape[0])
+    img = (rng.random(shape) * 10).astype(np.float32)
+    ks = [rng.standard_normal(K).astype(np.float32) for _ in range(3)]
+    lib = native.load()
+    a = torch.from_numpy(img).cuda()
+    b = torch.empty_like(a)
+    res = native.ctypes.c_void_p()
+    native.check(lib.mvd_separable_convolve_device(a.data_ptr(), b.data_ptr(), (native._F * 3)(*[native.fptr(k) for k in ks]),
+                                                   native.iarr([K] * 3), native.iarr(shape[::-1]), oob, -1.25, 0, None,
+                                                   native.ctypes.byref(res)))
+    torch.cuda.synchronize()
+    assert res.value == b.data_ptr()
+    _close(b.cpu().numpy(), O.separable_convolve(img, ks, oob, -1.25))
