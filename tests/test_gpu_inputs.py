@@ -192,6 +192,58 @@ def test_weight_overlap_matches_oracle(portions):
     assert wn.getMinOverlappingViews() == O.weight_overlap(ws, portions)[0] >= 1
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+@pytest.mark.parametrize("views", [1, 2, 5, 16])
+def test_normalize_weights_at_the_edges_of_the_float_sum(mode, views):
+    """Bit-equal at the limits of the float view sum (0 or 2^-24..2) and of the shared reciprocal
+    (sums from 2^100 on take the double pass), and for results beside a power of two."""
+    torch = pytest.importorskip("torch")
+    lib = native.load()
+    rng = np.random.default_rng(12)
+    f = np.float32
+    edge = np.array([0, -0.0, 2.0**-24, np.nextafter(f(2.0**-24), f(0)), 1, np.nextafter(f(1), f(0)),
+                     np.nextafter(f(1), f(2)), 2, np.nextafter(f(2), f(3)), 2.0**-47, 2.0**98, 2.0**100, 3e38], f)
+    n = 4001
+    ws = []
+    for _ in range(views):
+        w = rng.random(n).astype(f) * f(2)
+        pick = rng.random(n) < 0.6
+        w[pick] = edge[rng.integers(0, len(edge), pick.sum())]
+        small = rng.random(n) < 0.3  # voxels with the in-range values only
+        w[small] = edge[rng.integers(0, 8, small.sum())]
+        ws.append(w)
+    for osem in (1.0, 1.5, 1.7):
+        with np.errstate(all="ignore"):
+            want = (O.normalize_weights_virtual if mode == 0 else O.normalize_weights_precomputed)(ws, osem)
+        dws = [torch.from_numpy(w).cuda() for w in ws]
+        ptrs = (native.ctypes.c_void_p * views)(*[d.data_ptr() for d in dws])
+        native.check(lib.mvd_normalize_weights(ptrs, views, n, osem, mode, 0, None))
+        torch.cuda.synchronize()
+        for d, w in zip(dws, want):
+            np.testing.assert_array_equal(d.cpu().numpy(), w)
+
+
+@pytest.mark.parametrize("n", [1, 3, 127, 129, 40001])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_weight_overlap_of_slices(n, shift):
+    """Remainders of a lane's four voxels and of a warp's 128, and weights that start off a
+    16-byte boundary."""
+    torch = pytest.importorskip("torch")
+    from spim_registration_gb300 import WeightNormalizer
+
+    rng = np.random.default_rng(n)
+    ws = [np.where(rng.random(n) < 0.3, 0, rng.random(n)).astype(np.float32) for _ in range(3)]
+    portions = min(n, 7)
+    mn, avg = O.weight_overlap([w.reshape(1, 1, n) for w in ws], portions)
+    dws = [torch.zeros(n + shift, device="cuda")[shift:] for _ in ws]
+    for d, w in zip(dws, ws):
+        d.copy_(torch.from_numpy(w))
+    wn = WeightNormalizer([d.view(1, 1, n) for d in dws], num_portions=portions)
+    assert wn.process()
+    assert wn.getMinOverlappingViews() == mn
+    assert wn.getAvgOverlappingViews() == pytest.approx(avg, rel=1e-12)
+
+
 def test_raw_views_to_deconvolution_on_the_device():
     """Raw views + registrations -> resampled views and blending weights -> overlap statistics
     -> VIRTUAL normalisation with the average-overlap OSEM factor -> deconvolution from the
