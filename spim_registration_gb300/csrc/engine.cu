@@ -56,6 +56,39 @@ void keep_pool_memory(int dev) {
   done[dev] = true;
 }
 
+namespace {
+cudaMemPool_t call_pool(int dev) {
+  static std::mutex mu;
+  static std::map<int, cudaMemPool_t> pools;
+  std::lock_guard<std::mutex> lock(mu);
+  auto it = pools.find(dev);
+  if (it != pools.end()) return it->second;
+  cudaMemPoolProps props{};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = dev;
+  cudaMemPool_t pool;
+  MVD_CHECK(cudaMemPoolCreate(&pool, &props));
+  uint64_t keep = 64ull << 20;
+  const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) cudaMemPoolDestroy(pool);
+  MVD_CHECK(e);
+  return pools[dev] = pool;
+}
+}  // namespace
+
+CallBuf::CallBuf(int dev, size_t bytes, cudaStream_t s) : s_(s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  MVD_CHECK(cudaStreamIsCapturing(s, &st));
+  if (st == cudaStreamCaptureStatusNone)
+    MVD_CHECK(cudaMallocFromPoolAsync(&p_, bytes, call_pool(dev), s));
+  else
+    MVD_CHECK(cudaMallocAsync(&p_, bytes, s));
+}
+CallBuf::~CallBuf() {
+  if (p_) cudaFreeAsync(p_, s_);
+}
+
 void DevBuf::release() {
   if (p) {
     if (stream)

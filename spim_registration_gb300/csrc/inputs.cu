@@ -495,7 +495,8 @@ __global__ void normalize_deferred_kernel(WeightPtrs w, int nv, double osem, int
 // voxel a lane the kernel was issue-bound, 57.7 us at 4 views of 256x256x192; now 46.5 (4.3 TB/s).
 template <int NV, bool VEC>
 __global__ void weight_overlap_kernel(WeightPtrs w, long long n, long long chunk, int portions, long long span,
-                                      unsigned long long* __restrict__ portion_sum, int* __restrict__ min_count) {
+                                      unsigned long long* __restrict__ portion_sum,
+                                      int* __restrict__ max_missing) {  // views without weight at a voxel
   constexpr int nv = NV;
   const long long lo = blockIdx.x * span;
   const long long hi = lo + span < n ? lo + span : n;
@@ -562,7 +563,7 @@ __global__ void weight_overlap_kernel(WeightPtrs w, long long n, long long chunk
   }
   if (lane == 0 && cur >= 0 && acc) atomicAdd(portion_sum + cur, acc);
   const int m = __reduce_min_sync(0xffffffffu, local_min);
-  if (lane == 0) atomicMin(min_count, m);
+  if (lane == 0 && m < nv) atomicMax(max_missing, nv - m);
 }
 
 // f(std::integral_constant<int, nv>{}) for a view count 1..16
@@ -718,9 +719,8 @@ extern "C" int mvd_normalize_weights(float* const* weights, int num_views, long 
     // the deferred-voxel list, stream-ordered so that the call stays asynchronous
     Deferred def;
     def.cap = (unsigned long long)(n < (1LL << 22) ? n : (1LL << 22));
-    void* buf = nullptr;
-    MVD_CHECK(cudaMallocAsync(&buf, sizeof(unsigned long long) + def.cap * sizeof(long long), s));
-    def.count = static_cast<unsigned long long*>(buf);
+    const CallBuf buf(devCUDA, sizeof(unsigned long long) + def.cap * sizeof(long long), s);
+    def.count = buf.as<unsigned long long>();
     def.list = reinterpret_cast<long long*>(def.count + 1);
     MVD_CHECK(cudaMemsetAsync(def.count, 0, sizeof(unsigned long long), s));
     with_view_count(num_views, [&](auto nv) {
@@ -731,7 +731,6 @@ extern "C" int mvd_normalize_weights(float* const* weights, int num_views, long 
     normalize_deferred_kernel<<<152 * 4, 256, 0, s>>>(wp, num_views, osem, mode, def);
     MVD_CHECK(cudaGetLastError());
     count_launch();
-    MVD_CHECK(cudaFreeAsync(buf, s));
     return MVD_OK;
   } catch (const CudaError& e) {
     set_last_error(e.what());
@@ -761,14 +760,14 @@ extern "C" int mvd_weight_overlap(const float* const* weights, int num_views, lo
     }
     MVD_CHECK(cudaSetDevice(devCUDA));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // device scratch: the portion sums, then the minimum
-    const size_t bytes = (size_t)num_portions * sizeof(unsigned long long) + sizeof(int);
-    DevBuf scratch;
-    scratch.alloc(bytes);
+    // device scratch, all zero at first and read back in one copy: the portion sums, then the largest
+    // number of views missing at a voxel
+    std::vector<unsigned long long> sums(num_portions + 1);
+    const size_t bytes = sums.size() * sizeof(unsigned long long);
+    const CallBuf scratch(devCUDA, bytes, s);
     unsigned long long* d_sum = scratch.as<unsigned long long>();
-    int* d_min = reinterpret_cast<int*>(d_sum + num_portions);
-    MVD_CHECK(cudaMemsetAsync(d_sum, 0, (size_t)num_portions * sizeof(unsigned long long), s));
-    MVD_CHECK(cudaMemcpyAsync(d_min, &num_views, sizeof(int), cudaMemcpyHostToDevice, s));
+    int* d_missing = reinterpret_cast<int*>(d_sum + num_portions);
+    MVD_CHECK(cudaMemsetAsync(d_sum, 0, bytes, s));
     const int grid = grid_n(n);
     long long span = (n + grid - 1) / grid;
     span = (span + 127) / 128 * 128;
@@ -777,15 +776,15 @@ extern "C" int mvd_weight_overlap(const float* const* weights, int num_views, lo
     for (int v = 0; v < num_views; ++v) bits |= reinterpret_cast<uintptr_t>(weights[v]);
     with_view_count(num_views, [&](auto nv) {
       auto k = (bits & 15) ? weight_overlap_kernel<decltype(nv)::value, false> : weight_overlap_kernel<decltype(nv)::value, true>;
-      k<<<grid, 256, 0, s>>>(wp, n, chunk, num_portions, span, d_sum, d_min);
+      k<<<grid, 256, 0, s>>>(wp, n, chunk, num_portions, span, d_sum, d_missing);
     });
     MVD_CHECK(cudaGetLastError());
     count_launch();
-    std::vector<unsigned long long> sums(num_portions);
-    int mn = 0;
-    MVD_CHECK(cudaMemcpyAsync(sums.data(), d_sum, sums.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
-    MVD_CHECK(cudaMemcpyAsync(&mn, d_min, sizeof(int), cudaMemcpyDeviceToHost, s));
+    MVD_CHECK(cudaMemcpyAsync(sums.data(), d_sum, bytes, cudaMemcpyDeviceToHost, s));
     MVD_CHECK(cudaStreamSynchronize(s));
+    int missing;
+    std::memcpy(&missing, &sums[num_portions], sizeof(int));
+    const int mn = num_views - missing;
     // the reference averages the per-portion averages (WeightNormalizer.java:98-106)
     double avg = 0.0;
     for (int p = 0; p < num_portions; ++p) {

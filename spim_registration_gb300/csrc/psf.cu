@@ -288,11 +288,10 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
     const int chunks = std::max(1, (num_locations + per - 1) / per);
     const int nends = blocks_for(np);
     const size_t bb = (beads.size() * sizeof(Bead) + 15) / 16 * 16, eb = (size_t)nends * sizeof(float2);
-    void* buf = nullptr;
-    MVD_CHECK(cudaMallocAsync(&buf, bb + eb + (size_t)chunks * np * sizeof(float), s));
-    Bead* d_beads = static_cast<Bead*>(buf);
-    float2* d_ends = reinterpret_cast<float2*>(static_cast<char*>(buf) + bb);
-    float* d_part = reinterpret_cast<float*>(static_cast<char*>(buf) + bb + eb);
+    const CallBuf buf(devCUDA, bb + eb + (size_t)chunks * np * sizeof(float), s);
+    Bead* d_beads = buf.as<Bead>();
+    float2* d_ends = reinterpret_cast<float2*>(buf.as<char>() + bb);
+    float* d_part = reinterpret_cast<float*>(buf.as<char>() + bb + eb);
     if (num_locations > 0)
       MVD_CHECK(cudaMemcpyAsync(d_beads, beads.data(), beads.size() * sizeof(Bead), cudaMemcpyHostToDevice, s));
     extract_partial_kernel<<<dim3((items * 32 + kExtractThreads - 1) / kExtractThreads, chunks), kExtractThreads, 0, s>>>(
@@ -308,7 +307,6 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
       MVD_CHECK(cudaGetLastError());
       count_launch();
     }
-    MVD_CHECK(cudaFreeAsync(buf, s));
     return MVD_OK;
   } catch (const CudaError& e) {
     set_last_error(e.what());

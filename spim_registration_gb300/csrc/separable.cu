@@ -302,14 +302,18 @@ int walk_segment(int n, long long warps_per_segment, long long resident, int R) 
   return best;
 }
 
-// warps of a kernel resident at once on the current device (kWalkThreads per block)
-template <class K>
-long long resident_warps(K kernel) {
-  int dev = 0, sms = 0, blocks = 0;
-  MVD_CHECK(cudaGetDevice(&dev));
-  MVD_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  MVD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kWalkThreads, 0));
-  return (long long)sms * std::max(1, blocks) * (kWalkThreads / 32);
+// warps of a kernel resident at once on the GPU (kWalkThreads per block).  A property of the compiled
+// kernel, asked once: the three queries took 1 us of each pass's launch.
+template <auto kernel>
+long long resident_warps() {
+  static const long long warps = [] {
+    int dev = 0, sms = 0, blocks = 0;
+    MVD_CHECK(cudaGetDevice(&dev));
+    MVD_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    MVD_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, kWalkThreads, 0));
+    return (long long)sms * std::max(1, blocks) * (kWalkThreads / 32);
+  }();
+  return warps;
 }
 
 template <int R>
@@ -322,7 +326,7 @@ void launch_walk(int axis, const float* in, float* out, int w, int h, int d, con
   if (outer > 65535 || (n + kCH - 1) / kCH > 65535) throw std::invalid_argument("image too large for the y/z passes");
   const long long positions = (long long)w * outer;
   const long long blocks = (positions + kWalkThreads - 1) / kWalkThreads;
-  int seg = walk_segment(n, blocks * (kWalkThreads / 32), resident_warps(sep_walk_kernel<R>), R);
+  int seg = walk_segment(n, blocks * (kWalkThreads / 32), resident_warps<sep_walk_kernel<R>>(), R);
   seg = std::max(seg, (n + 65534) / 65535);
   sep_walk_kernel<R><<<dim3((unsigned)blocks, (n + seg - 1) / seg), kWalkThreads, 0, s>>>(in, out, w, positions, n, sa, so,
                                                                                        seg, t, oob, value);
@@ -334,7 +338,7 @@ template <int R, int P>
 void launch_x_of(const float* in, float* out, int w, long long rows, const Taps& t, int oob, float value, cudaStream_t s) {
   const int xt = (w + 32 * P - 1) / (32 * P);
   // two waves of warps; at most 64 rows each
-  const long long warps = 2 * resident_warps(sep_x_kernel<R, P>);
+  const long long warps = 2 * resident_warps<sep_x_kernel<R, P>>();
   const int run = (int)std::max(1LL, std::min(64LL, rows * xt / warps));
   const long long blocks = ((rows + run - 1) / run * xt + kXThreads / 32 - 1) / (kXThreads / 32);
   if (blocks > 0x7fffffffLL) throw std::invalid_argument("image too large for the x pass");

@@ -19,8 +19,8 @@ def _torch():
     return torch
 
 
-def extract_psf_local(img, locations_xyz, psf_size_xyz, normalize=False, device: int = 0) -> np.ndarray:
-    """ExtractPSF.extractPSFLocal (:374-415), optionally followed by ExtractPSF.normalize (:298-316)."""
+def _extract(img, locations_xyz, psf_size_xyz, normalize: bool, device: int):
+    """The extracted PSF on the view's device."""
     torch = _torch()
     lib = native.load()
     t = img if getattr(img, "is_cuda", False) else torch.from_numpy(
@@ -34,7 +34,12 @@ def extract_psf_local(img, locations_xyz, psf_size_xyz, normalize=False, device:
                                      loc.ctypes.data_as(ctypes.POINTER(ctypes.c_double)), len(loc),
                                      native.iarr([px, py, pz]), out.data_ptr(), int(bool(normalize)),
                                      t.device.index, ctypes.c_void_p(st.cuda_stream)))
-    return out.cpu().numpy()
+    return out
+
+
+def extract_psf_local(img, locations_xyz, psf_size_xyz, normalize=False, device: int = 0) -> np.ndarray:
+    """ExtractPSF.extractPSFLocal (:374-415), optionally followed by ExtractPSF.normalize (:298-316)."""
+    return _extract(img, locations_xyz, psf_size_xyz, normalize, device).cpu().numpy()
 
 
 def transformed_psf_size(psf_size_xyz, model):
@@ -48,22 +53,26 @@ def transformed_psf_size(psf_size_xyz, model):
     return tuple(dims), tuple(off)
 
 
-def transform_psf(psf: np.ndarray, model, device: int = 0) -> np.ndarray:
-    """ExtractPSF.transformPSF + transform (:325-372, :417-464): the PSF resampled by the view's
-    model into an odd-sized box whose centre is the PSF's centre voxel."""
+def _transform(t, model, device: int):
+    """The PSF on the device (float32, contiguous), transformed there."""
     torch = _torch()
     lib = native.load()
-    psf = np.ascontiguousarray(psf, dtype=np.float32)
-    pz, py, px = psf.shape
+    pz, py, px = t.shape
     (nx, ny, nz), off = transformed_psf_size((px, py, pz), model)
-    t = torch.from_numpy(psf).to(f"cuda:{device}")
     out = torch.empty((nz, ny, nx), dtype=torch.float32, device=t.device)
     st = torch.cuda.current_stream(t.device)
     native.check(lib.mvd_transform_psf(t.data_ptr(), native.iarr([px, py, pz]),
                                        (ctypes.c_double * 12)(*np.asarray(model, dtype=np.float64).ravel()),
                                        native.iarr([nx, ny, nz]), (ctypes.c_double * 3)(*off), out.data_ptr(),
                                        device, ctypes.c_void_p(st.cuda_stream)))
-    return out.cpu().numpy()
+    return out
+
+
+def transform_psf(psf: np.ndarray, model, device: int = 0) -> np.ndarray:
+    """ExtractPSF.transformPSF + transform (:325-372, :417-464): the PSF resampled by the view's
+    model into an odd-sized box whose centre is the PSF's centre voxel."""
+    t = _torch().from_numpy(np.ascontiguousarray(psf, dtype=np.float32)).to(f"cuda:{device}")
+    return _transform(t, model, device).cpu().numpy()
 
 
 def make_same_size(img: np.ndarray, size_xyz) -> np.ndarray:
@@ -90,10 +99,12 @@ class ExtractPSF:
 
     def extractNextImg(self, img, viewId, model, locations_xyz, psf_size_xyz):
         """ExtractPSF.extractNextImg (:277-296)."""
-        original = extract_psf_local(img, locations_xyz, psf_size_xyz, normalize=True, device=self.device)
+        original = _extract(img, locations_xyz, psf_size_xyz, True, self.device)
         self.viewIds.append(viewId)
-        self.pointSpreadFunctions[viewId] = transform_psf(original, model, self.device)
-        self.originalPSFs[viewId] = original
+        # transformed where it lies; both copied to the host behind the two kernels' one wait
+        transformed = _transform(original.to(f"cuda:{self.device}"), model, self.device)
+        self.pointSpreadFunctions[viewId] = transformed.cpu().numpy()
+        self.originalPSFs[viewId] = original.cpu().numpy()
 
     def getPSFMap(self):
         return self.pointSpreadFunctions
