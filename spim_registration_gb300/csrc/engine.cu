@@ -1069,15 +1069,24 @@ __device__ __forceinline__ void pair_add(float& hi, float& lo, float bh, float b
 // HBM speed, so each thread carries its sum as a float pair (the voxel's view sum by exact
 // two-sums, times 1/c as a pair), flushed into a double every 16 voxels.  The reference's
 // RealSum is itself order-dependent; each pair chunk is accurate to ~2^-43.
-__global__ void first_iteration_kernel(ViewPtrs v, int nviews, long long n, double* out) {
+//
+// The views' loads of a voxel go out before the first is used, and one wave of blocks walks the volume:
+// the double sums over a block's threads are FP64 work per thread, not per voxel (at 16 blocks an SM
+// they took most of the 51 us at 3 views of 203x157x91).
+template <int NV>
+__global__ void __launch_bounds__(256, 6) first_iteration_kernel(ViewPtrs v, long long n, double* out) {
   float acc_hi = 0.f, acc_lo = 0.f;
   double total = 0.0;
   unsigned long long cnt = 0;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+    float xs[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) xs[k] = __ldg(v.p[k] + i);
     float s_hi = 0.f, s_lo = 0.f;
     int c = 0;
-    for (int k = 0; k < nviews; ++k) {
-      const float x = __ldg(v.p[k] + i);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      const float x = xs[k];
       if (x > 0.f) {
         float e;
         two_sum(s_hi, x, s_hi, e);
@@ -1104,7 +1113,14 @@ void dev_first_iteration(const float* const* views, int nviews, long long n, dou
   ViewPtrs vp{};
   if (nviews > 16) throw std::invalid_argument("at most 16 views");
   for (int i = 0; i < nviews; ++i) vp.p[i] = views[i];
-  first_iteration_kernel<<<grid_for(n), 256, 0, s>>>(vp, nviews, n, out);
+  using Kernel = void (*)(ViewPtrs, long long, double*);
+  static constexpr Kernel kernels[17] = {
+      first_iteration_kernel<1>,  first_iteration_kernel<1>,  first_iteration_kernel<2>,  first_iteration_kernel<3>,
+      first_iteration_kernel<4>,  first_iteration_kernel<5>,  first_iteration_kernel<6>,  first_iteration_kernel<7>,
+      first_iteration_kernel<8>,  first_iteration_kernel<9>,  first_iteration_kernel<10>, first_iteration_kernel<11>,
+      first_iteration_kernel<12>, first_iteration_kernel<13>, first_iteration_kernel<14>, first_iteration_kernel<15>,
+      first_iteration_kernel<16>};
+  kernels[nviews]<<<std::min(grid_for(n), 152 * 6), 256, 0, s>>>(vp, n, out);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }
@@ -1214,41 +1230,66 @@ void dev_paste_block(const float* block, int bx, int by, int bz, int lx, int ly,
   count_launch();
 }
 
+//
+// A warp takes a row of x at a time, four loads of each volume per lane in flight, so that y and z need
+// one division a row and one set of atomics a block.  A voxel per thread cost three 64-bit divisions at
+// every voxel with data: 73 us at 203x157x91 (23 MB).
 __global__ void data_box_kernel(const float* __restrict__ img, const float* __restrict__ w, int nx, int ny, int nz,
                                 int* box) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
-  const long long n = (long long)nx * ny * nz;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    if (__ldg(img + i) > 0.f || __ldg(w + i) > 0.f) {
-      const int c[3] = {(int)(i % nx), (int)((i / nx) % ny), (int)(i / ((long long)nx * ny))};
+  const long long rows = (long long)ny * nz;
+  for (long long r = blockIdx.x * (long long)warps + warp; r < rows; r += (long long)gridDim.x * warps) {
+    const float* pi = img + r * nx;
+    const float* pw = w + r * nx;
+    bool any = false;
+    for (int x0 = lane; x0 < nx; x0 += 128) {
+      float a[4], b[4];
 #pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        lo[d] = min(lo[d], c[d]);
-        hi[d] = max(hi[d], c[d]);
+      for (int e = 0; e < 4; ++e) {
+        const bool in = x0 + 32 * e < nx;
+        a[e] = in ? __ldg(pi + x0 + 32 * e) : 0.f;
+        b[e] = in ? __ldg(pw + x0 + 32 * e) : 0.f;
       }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (a[e] > 0.f || b[e] > 0.f) {
+          any = true;
+          lo[0] = min(lo[0], x0 + 32 * e);
+          hi[0] = max(hi[0], x0 + 32 * e);
+        }
+    }
+    if (any) {
+      const int z = (int)(r / ny), y = (int)(r - (long long)z * ny);
+      lo[1] = min(lo[1], y);
+      hi[1] = max(hi[1], y);
+      lo[2] = min(lo[2], z);
+      hi[2] = max(hi[2], z);
     }
   }
+  __shared__ int s_box[6];
+  if (threadIdx.x < 6) s_box[threadIdx.x] = threadIdx.x < 3 ? INT_MAX : -1;
+  __syncthreads();
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      lo[d] = min(lo[d], __shfl_xor_sync(0xffffffffu, lo[d], o));
-      hi[d] = max(hi[d], __shfl_xor_sync(0xffffffffu, hi[d], o));
+    const int l = __reduce_min_sync(0xffffffffu, lo[d]), h = __reduce_max_sync(0xffffffffu, hi[d]);
+    if (lane == 0 && h >= 0) {
+      atomicMin(s_box + d, l);
+      atomicMax(s_box + 3 + d, h);
     }
   }
-  if ((threadIdx.x & 31) == 0) {
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      if (hi[d] >= 0) {
-        atomicMin(box + d, lo[d]);
-        atomicMax(box + 3 + d, hi[d]);
-      }
-    }
+  __syncthreads();
+  if (threadIdx.x < 6 && s_box[3] >= 0) {
+    if (threadIdx.x < 3)
+      atomicMin(box + threadIdx.x, s_box[threadIdx.x]);
+    else
+      atomicMax(box + threadIdx.x, s_box[threadIdx.x]);
   }
 }
 
 void dev_data_box(const float* img, const float* w, int nx, int ny, int nz, int* box, cudaStream_t s) {
-  data_box_kernel<<<grid_for((long long)nx * ny * nz), 256, 0, s>>>(img, w, nx, ny, nz, box);
+  const long long blocks = std::min(((long long)ny * nz + 7) / 8, 152LL * 8);  // one wave of 256 threads
+  data_box_kernel<<<(int)blocks, 256, 0, s>>>(img, w, nx, ny, nz, box);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }
