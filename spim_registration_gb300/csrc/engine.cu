@@ -561,13 +561,34 @@ size_t pair_plane_smem(int m, int ty) {
 }
 
 // CTA size of the plane passes: 128 registers per thread, so 512 threads per SM over the CTAs that
-// fit its shared memory; no more than a stage has work for.
+// share one (that fit its shared memory, and that there are: 270 planes of 128x128x64 took 13.2 us with
+// 128 threads, 12.3 with 256); no more than a stage has work for, but 128 for the gather and the
+// epilogue (40x32x24: 8.8 us with 64, 8.5).
 int pair_plane_threads(const PairShape& s, size_t smem, long long planes) {
-  const int ctas = pair_ctas_per_sm(smem);
+  const int ctas = (int)std::min<long long>(pair_ctas_per_sm(smem), (planes + 151) / 152);
   int t = ctas >= 4 ? 128 : ctas >= 2 ? 256 : 512;
-  if (planes <= 152) t = 512;  // at most one CTA per SM anyway
   const int work = std::max(std::max(s.ty / 2 * s.r1x, s.ty / 2 * s.r0x), std::max(s.nunits * (s.r1y / 2), s.pc * s.r0y));
-  return std::max(64, std::min(t, (work + 31) / 32 * 32));
+  return std::max(128, std::min(t, (work + 31) / 32 * 32));
+}
+
+// CTA size of the z pass: 640 threads per SM in all, so what counts is how well a size divides the
+// stages' items (their points x 8 pencil pairs), per CTA that shares the SM: 128 threads, or 160 or 64
+// where that is an eighth better by this measure, and no more than one step takes.  us per pass with
+// 64 / 128 / 160 threads: 120 points 11.8 / 13.8 / 14.3 (203x157x91, 3 views); 320 points 328 / 274 / 259
+// (512x512x256, 4 views); 240 and 216 points 63.0 / 51.1 / 52.1 (256x256x192, 4 views); 90 and 72 points
+// 7.5 / 6.5 / 9.2 (128x128x64, 2 views).  96 threads were never the best.
+int pair_z_threads(const PairShape& s) {
+  const int na = s.bz * s.cz * kPairChunk, nb = s.bz > 1 ? s.az * s.cz * kPairChunk : 0, nc = s.az * s.bz * kPairChunk;
+  const int most = std::max({na, nb, nc});
+  if (most <= 128) return most <= 64 ? 64 : 128;
+  const int fit = std::max(1, (int)(227 * 1024 / (((size_t)s.tz * kPairChunk + s.tz) * sizeof(float4) + 1024)));
+  auto cost = [&](int t) {
+    auto steps = [t](int n) { return (n + t - 1) / t; };
+    return (2.0 * steps(na) + 2.0 * steps(nb) + 1.5 * steps(nc)) / std::min(640 / t, fit);
+  };
+  const double c64 = cost(64), c128 = cost(128), c160 = cost(160);
+  if (std::min(c64, c160) > 0.88 * c128) return 128;
+  return c64 < c160 ? 64 : 160;
 }
 
 // Tile shape and tables for the pair kernels; false when no shape fits (a kernel too large for
@@ -599,7 +620,7 @@ bool plan_pairs(ConvPlan& p, int nx, int ny, int nz, int kx, int ky, int kz, con
           return std::ceil(items / (152.0 * conc)) * conc * work;
         };
         const double cost = (4.0 * f * waves(nt * c.a.T, ctas, plane) +
-                             1.8 * waves(nt * std::ceil(plane / (2.0 * kPairChunk)), 2.0, 2.0 * kPairChunk * c.a.T)) *
+                             1.8 * waves(nt * std::ceil(plane / (2.0 * kPairChunk)), 4.0, 2.0 * kPairChunk * c.a.T)) *
                             (1.0 + 1e-3 * nt);
         if (cost < best) {
           best = cost;
@@ -655,6 +676,7 @@ bool plan_pairs(ConvPlan& p, int nx, int ny, int nz, int kx, int ky, int kz, con
   p.z_chunks = (plane + kPairChunk - 1) / kPairChunk;
   p.pair_threads = opt.threads > 0 ? opt.threads : pair_plane_threads(s, p.smem_pair, (long long)p.tiles.size() * s.tz);
   p.threads_plane = p.pair_threads;
+  p.pair_z_threads = pair_z_threads(s);
   return true;
 }
 

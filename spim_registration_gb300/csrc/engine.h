@@ -137,6 +137,7 @@ struct ConvPlan {
   bool paired = false;
   PairShape ps{};
   int pair_threads = 0;                // CTA size of the plane passes
+  int pair_z_threads = 0;              // and of the z pass
   int z_chunks = 0;                    // pencil-pair chunks of a tile
   size_t smem_pair = 0, smem_pair_z = 0;
   DevBuf d_pair;                       // tiles, one full tile, roots and column units in one block

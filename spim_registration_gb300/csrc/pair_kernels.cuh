@@ -37,8 +37,8 @@
 namespace mvd {
 
 constexpr int kPairThreads = 512;  // largest plane CTA; 128 registers per thread
-constexpr int kPairZThreads = 320;  // two CTAs per SM at 96 registers
-constexpr int kPairChunk = 16;  // pencil pairs per z CTA: 256-byte rows
+constexpr int kPairZThreads = 160;  // at most; 640 threads per SM at 96 registers
+constexpr int kPairChunk = 8;  // pencil pairs per z CTA: 128-byte rows
 
 #define MVD_PAIR_X0(X) X(2) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(16)
 #define MVD_PAIR_X1(X) X(2) X(3) X(4) X(5) X(6) X(8) X(9) X(10) X(12) X(15) X(16)
@@ -632,7 +632,10 @@ pair_inv(const TileDesc* __restrict__ tiles, int ntiles, const float4* __restric
 }
 
 // ------------------------------------------------------------------------------------------
-// z pass: kPairChunk pencil pairs per CTA
+// z pass: kPairChunk pencil pairs per CTA.  A CTA's stages wait on one another, so what keeps the SM busy
+// is the number of CTAs that share it: 8 pairs and 64 to 160 threads (4 to 10 CTAs) against 16 pairs and
+// 320 threads (2) took 260 / 281 us at 512x512x256 (4 views), 50.8 / 58.0 at 256x256x192, 11.8 / 15.1 at
+// 203x157x91.
 // ------------------------------------------------------------------------------------------
 // Lengths are A x B x C (B = 1: two stages) with radices of at most 10 (C: 8).  The middle stage C holds
 // its points and the kernel spectrum's values of the same positions, which are loaded before the
@@ -645,7 +648,7 @@ template <int R>
 __device__ __forceinline__ void pair_za_fwd(const PairShape& s, const float4* __restrict__ g, int plane, int count,
                                             float4* sm) {
   const int NR = s.bz * s.cz, nb = NR * kPairChunk;
-  for (int b = threadIdx.x; b < nb; b += kPairZThreads) {
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     const int j = b / kPairChunk, i = b % kPairChunk;
     if (i >= count) continue;
     C2 v[R];
@@ -662,7 +665,7 @@ __device__ __forceinline__ void pair_za_fwd(const PairShape& s, const float4* __
 template <int R, bool INV>
 __device__ __forceinline__ void pair_zb(const PairShape& s, float4* sm, const float2* tw) {
   const int C = s.cz, nb = s.az * C * kPairChunk;
-  for (int b = threadIdx.x; b < nb; b += kPairZThreads) {
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     const int kj = b / kPairChunk, i = b % kPairChunk;
     const int k0 = kj / C, p0 = k0 * (R * C) + kj - k0 * C;
     float4* p = sm + p0 * kPairChunk + i;
@@ -698,7 +701,7 @@ __device__ __forceinline__ void pair_zc(const PairShape& s, float4* __restrict__
   int b = threadIdx.x;
   load(b);
   __syncthreads();  // the stage before (or the tables) is complete; the loads are in flight meanwhile
-  for (; b < nb; b += kPairZThreads, load(b)) {
+  for (; b < nb; b += blockDim.x, load(b)) {
     if (i >= count) continue;
     const int kb = b / kPairChunk;
     float4* p = sm + (kb * R) * kPairChunk + i;
@@ -729,7 +732,7 @@ template <int R>
 __device__ __forceinline__ void pair_za_inv(const PairShape& s, float4* __restrict__ g, int plane, int count,
                                             const float4* sm, int z0, int z1) {
   const int NR = s.bz * s.cz, nb = NR * kPairChunk;
-  for (int b = threadIdx.x; b < nb; b += kPairZThreads) {
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     const int j = b / kPairChunk, i = b % kPairChunk;
     if (i >= count) continue;
     const float4* p = sm + j * kPairChunk + i;
@@ -754,7 +757,7 @@ __device__ __forceinline__ void pair_za_inv(const PairShape& s, float4* __restri
 // Item b: blocks of `block` chunks, each swept over every tile before the next, so that a block's
 // kernel spectrum is read from L2 by every tile but the first.
 template <bool CONV>
-__global__ void __launch_bounds__(kPairZThreads, 2)
+__global__ void __launch_bounds__(kPairZThreads, 4)
 pair_z(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ spec, const float4* __restrict__ otf,
        const __grid_constant__ PairShape s, int nchunks, int block, float scale) {
   extern __shared__ float4 sm4[];

@@ -3,16 +3,16 @@
 
 namespace mvd {
 
-// Chunks of a block: 32 chunks (8 KB rows per slice) keep the block's kernel spectrum in L2 while
+// Chunks of a block: 64 chunks (8 KB rows per slice) keep the block's kernel spectrum in L2 while
 // every tile reads it, and each tile's reads contiguous over the block.
-constexpr int kPairZBlock = 32;
+constexpr int kPairZBlock = 64;
 
 template <bool CONV>
 static void launch(const ConvPlan& p, TileSet set, float2* spec, const float2* otf, float scale, cudaStream_t s) {
   const PairTiles t = pair_tiles(p, set);
   auto k = pair_z<CONV>;
   set_smem(k, p.smem_pair_z);
-  k<<<t.n * p.z_chunks, kPairZThreads, p.smem_pair_z, s>>>(t.t, t.n, reinterpret_cast<float4*>(spec),
+  k<<<t.n * p.z_chunks, p.pair_z_threads, p.smem_pair_z, s>>>(t.t, t.n, reinterpret_cast<float4*>(spec),
                                                            reinterpret_cast<const float4*>(otf), p.ps, p.z_chunks,
                                                            kPairZBlock, scale);
   MVD_CHECK(cudaGetLastError());

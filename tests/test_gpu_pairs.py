@@ -49,6 +49,26 @@ def test_device_convolution_matches_fp64(shape, kshape, mode, value):
     assert rel_max(got, O.conv_extended(x, k, mode, value)) < TOL
 
 
+@pytest.mark.parametrize("nz,kz", [(5, 3), (20, 5), (60, 13), (78, 13), (108, 13), (120, 31), (136, 15), (212, 29),
+                                   (224, 31), (260, 61)])
+def test_z_lengths_match_fp64(nz, kz):
+    """The z pass at lengths of every CTA size (64, 128 and 160 threads) and their remainders, with
+    planes that end in the middle of a chunk of pencil pairs."""
+    torch = pytest.importorskip("torch")
+    lib = native.load()
+    rng = np.random.default_rng(nz)
+    shape, kshape = (nz, 70, 76), (kz, 5, 7)
+    x = (rng.random(shape) * 100).astype(np.float32)
+    k = rng.random(kshape).astype(np.float32)
+    k /= k.sum()
+    xd, kd = torch.from_numpy(x).cuda(), torch.from_numpy(k).cuda()
+    out = torch.full_like(xd, float("nan"))
+    torch.cuda.synchronize()
+    native.check(lib.mvd_convolve3d_device(xd.data_ptr(), out.data_ptr(), native.iarr(shape[::-1]), kd.data_ptr(),
+                                           native.iarr(kshape[::-1]), 0, 0.0, 0, None))
+    assert rel_max(out.cpu().numpy(), O.conv_extended(x, k, O.MIRROR, 0.0)) < TOL
+
+
 @pytest.mark.parametrize("shape,lo,hi", [
     ((61, 53, 47), (0, 0, 0), (61, 53, 47)),
     ((64, 56, 48), (3, 5, 2), (60, 51, 47)),   # data boxes at odd positions, aligned rows
