@@ -245,6 +245,24 @@ inline void set_smem(K kernel, size_t bytes) {
   set_smem_raw(reinterpret_cast<const void*>(kernel), bytes);
 }
 
+// Launches a kernel that may start before the kernel ahead of it in the stream has finished; it waits
+// for that one itself (wait_for_passes_ahead) before it touches what another kernel writes or reads.
+// Behind anything but a kernel, and in a plain launch, the stream's order holds as usual.
+template <class... P, class... A>
+inline void launch_after(void (*k)(P...), int grid, int threads, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)grid);
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  MVD_CHECK(cudaLaunchKernelEx(&c, k, static_cast<P>(args)...));
+}
+
 // Forward plane pass gathering from a (vx, vy, vz) volume with a constant border value; and the
 // forward-only, scaled z pass (kernel spectra; spectra of the PSF gradient).
 void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float* vol, int vx, int vy, int vz,

@@ -8,8 +8,7 @@ static void launch(const ConvPlan& p, TileSet set, const Gather& g, float2* spec
   const PairTiles t = pair_tiles(p, set);
   auto k = pair_fwd<Gather>;
   set_smem(k, p.smem_pair);
-  k<<<t.n * p.ps.tz, p.pair_threads, p.smem_pair, s>>>(t.t, t.n, reinterpret_cast<float4*>(spec), g, p.ps);
-  MVD_CHECK(cudaGetLastError());
+  launch_after(k, t.n * p.ps.tz, p.pair_threads, p.smem_pair, s, t.t, t.n, reinterpret_cast<float4*>(spec), g, p.ps);
   count_launch();
 }
 

@@ -8,8 +8,8 @@ static void launch(const ConvPlan& p, const float2* spec, const Epi& e, cudaStre
   const PairTiles t = pair_tiles(p, TileSet::All);
   auto k = pair_inv<Epi>;
   set_smem(k, p.smem_pair);
-  k<<<t.n * p.tiles[0].ez, p.pair_threads, p.smem_pair, s>>>(t.t, t.n, reinterpret_cast<const float4*>(spec), e, p.ps);
-  MVD_CHECK(cudaGetLastError());
+  launch_after(k, t.n * p.tiles[0].ez, p.pair_threads, p.smem_pair, s, t.t, t.n, reinterpret_cast<const float4*>(spec),
+               e, p.ps);
   count_launch();
 }
 

@@ -85,6 +85,12 @@ __device__ __forceinline__ C2 ldg_c2_early(const float4* p) {  // not moved acro
 }
 
 
+// The three passes are launched so that a pass may start before the one ahead of it in the stream has
+// finished (launch_after): each lets the next one start at once, copies its tables, which no pass
+// writes, and waits here for the passes ahead to complete before it reads or writes anything else.
+__device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunchCompletion(); }
+__device__ __forceinline__ void wait_for_passes_ahead() { cudaGridDependencySynchronize(); }
+
 // work item b of a plane pass: slice by slice, every tile of a slice before the next slice (the
 // halos that neighbouring tiles share are then gathered from L2)
 __device__ __forceinline__ void plane_item(int b, int ntiles, int& tile, int& z) {
@@ -319,6 +325,13 @@ pair_fwd(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ sp
   plane_item(blockIdx.x, ntiles, ti, z);
   const TileDesc t = tiles[ti];
   float4* out = spec + t.spec_off / 2 + (long long)z * s.ty * s.pc;
+  float4* const tab = sm + (s.ty >> 1) * s.pitch;
+  const float2* const twx = reinterpret_cast<const float2*>(tab);
+  const float2* const twy = reinterpret_cast<const float2*>(tab + s.tab_y);
+  const int4* const units = reinterpret_cast<const int4*>(tab + s.tab_units);
+  let_next_start();
+  copy_table(tab, s.tab, s.ntab);
+  wait_for_passes_ahead();
   // a slice of one value: the extension outside the data box, and the slices past the last one
   // that the effective region reaches (any finite value serves there)
   float cval = 0.f;
@@ -329,11 +342,6 @@ pair_fwd(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ sp
     for (int i = threadIdx.x; i < s.ty * s.pc; i += blockDim.x) out[i] = make_float4(i == 0 ? dc : 0.f, 0.f, 0.f, 0.f);
     return;
   }
-  float4* const tab = sm + (s.ty >> 1) * s.pitch;
-  const float2* const twx = reinterpret_cast<const float2*>(tab);
-  const float2* const twy = reinterpret_cast<const float2*>(tab + s.tab_y);
-  const int4* const units = reinterpret_cast<const int4*>(tab + s.tab_units);
-  copy_table(tab, s.tab, s.ntab);
   {
     PairGather<Gather> pg{PairRows<Gather>(gather, t.oz + z, t.ox, t.oy, 2 * s.m, s.ty)};
     pg.ox = t.ox;
@@ -586,16 +594,18 @@ pair_inv(const TileDesc* __restrict__ tiles, int ntiles, const float4* __restric
   int ti, z;
   plane_item(blockIdx.x, ntiles, ti, z);
   const TileDesc t = tiles[ti];
+  float4* const tab = sm + (s.ty >> 1) * s.pitch;
   epi.acc_init();
+  let_next_start();
+  if (z < t.ez) copy_table(tab, s.tab, s.ntab);
+  wait_for_passes_ahead();
   if (z < t.ez) {
     z += t.hz;
     const float4* in = spec + t.spec_off / 2 + (long long)z * s.ty * s.pc;
     const int q0 = t.hy >> 1, q1 = (t.hy + t.ey + 1) >> 1;
     float4* rows = sm + q0 * s.pitch;
-    float4* const tab = sm + (s.ty >> 1) * s.pitch;
     const float2* const twx = reinterpret_cast<const float2*>(tab);
     const int4* const units = reinterpret_cast<const int4*>(tab + s.tab_units);
-    copy_table(tab, s.tab, s.ntab);
     switch (s.r1y) { MVD_PAIR_Y1(MVD_CASE_Y1I) }
     __syncthreads();
     switch (s.r0y) { MVD_PAIR_Y0(MVD_CASE_Y0I) }
@@ -775,7 +785,9 @@ pair_z(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ spec
   // roots of the second stage by position, then of the third (the same table when B = 1)
   const float2* const tw = reinterpret_cast<const float2*>(sm + s.tz * kPairChunk);
   const float2* const twc = reinterpret_cast<const float2*>(sm + s.tz * kPairChunk + s.tab_c);
+  let_next_start();
   copy_table(sm + s.tz * kPairChunk, s.tabz, s.ntabz);
+  wait_for_passes_ahead();
   switch (s.az) { MVD_PAIR_Z(MVD_CASE_ZAF) }
   if (s.bz > 1) {
     __syncthreads();

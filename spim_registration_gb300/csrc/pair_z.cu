@@ -12,10 +12,8 @@ static void launch(const ConvPlan& p, TileSet set, float2* spec, const float2* o
   const PairTiles t = pair_tiles(p, set);
   auto k = pair_z<CONV>;
   set_smem(k, p.smem_pair_z);
-  k<<<t.n * p.z_chunks, p.pair_z_threads, p.smem_pair_z, s>>>(t.t, t.n, reinterpret_cast<float4*>(spec),
-                                                           reinterpret_cast<const float4*>(otf), p.ps, p.z_chunks,
-                                                           kPairZBlock, scale);
-  MVD_CHECK(cudaGetLastError());
+  launch_after(k, t.n * p.z_chunks, p.pair_z_threads, p.smem_pair_z, s, t.t, t.n, reinterpret_cast<float4*>(spec),
+               reinterpret_cast<const float4*>(otf), p.ps, p.z_chunks, kPairZBlock, scale);
   count_launch();
 }
 
