@@ -45,36 +45,16 @@ __device__ __forceinline__ int mirror_single_i(int i, int n) {
   return m < n ? m : period - m;
 }
 
-// NLinearInterpolator over Views.extendMirrorSingle(img) at the real position t; Index is the
-// voxel index type (32-bit when the view holds fewer than 2^31 voxels)
-template <class Index>
-__device__ __forceinline__ float trilinear_mirror(const float* __restrict__ img, int sx, int sy, int sz, float tx,
-                                                  float ty, float tz) {
-  const float fx0 = floorf(tx), fy0 = floorf(ty), fz0 = floorf(tz);
-  const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-  const float ax = tx - fx0, ay = ty - fy0, az = tz - fz0;
-  float val[8];
-  if (x0 >= 0 && y0 >= 0 && z0 >= 0 && x0 < sx - 1 && y0 < sy - 1 && z0 < sz - 1) {
-    // all eight corners inside: fixed distances from one (nearly every voxel; the index mirroring of
-    // the general case took half of the kernel's instructions: 104 -> 80 us per 256x256x192 view)
-    const float* p = img + ((Index)z0 * sy + y0) * sx + x0;
-    const float* q = p + (Index)sy * sx;
-    val[0] = __ldg(p);
-    val[1] = __ldg(p + 1);
-    val[2] = __ldg(p + sx);
-    val[3] = __ldg(p + sx + 1);
-    val[4] = __ldg(q);
-    val[5] = __ldg(q + 1);
-    val[6] = __ldg(q + sx);
-    val[7] = __ldg(q + sx + 1);
-  } else {
-    const int xs[2] = {mirror_single_i(x0, sx), mirror_single_i(x0 + 1, sx)};
-    const int ys[2] = {mirror_single_i(y0, sy), mirror_single_i(y0 + 1, sy)};
-    const int zs[2] = {mirror_single_i(z0, sz), mirror_single_i(z0 + 1, sz)};
-#pragma unroll
-    for (int c = 0; c < 8; ++c)
-      val[c] = __ldg(img + ((Index)zs[(c >> 2) & 1] * sy + ys[(c >> 1) & 1]) * sx + xs[c & 1]);
-  }
+// A view and its size.  Off is the type of byte offsets into it: 32 bits where the view holds fewer than
+// 2^30 voxels, so that a corner's address is one of four base pointers, the same in every thread, plus a
+// 32-bit register.
+struct View {
+  const float* img;
+  int sx, sy, sz;
+};
+
+// The trilinear sum of the eight corners, x fastest
+__device__ __forceinline__ float corner_sum(const float* val, float ax, float ay, float az) {
   float acc = 0.f;
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
@@ -83,6 +63,22 @@ __device__ __forceinline__ float trilinear_mirror(const float* __restrict__ img,
     acc += w * val[c];
   }
   return acc;
+}
+
+// NLinearInterpolator over Views.extendMirrorSingle(img) at a real position whose corners may lie
+// outside
+template <class Off>
+__device__ __noinline__ float trilinear_mirror(View v, float tx, float ty, float tz) {
+  const float fx0 = floorf(tx), fy0 = floorf(ty), fz0 = floorf(tz);
+  const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
+  const int xs[2] = {mirror_single_i(x0, v.sx), mirror_single_i(x0 + 1, v.sx)};
+  const int ys[2] = {mirror_single_i(y0, v.sy), mirror_single_i(y0 + 1, v.sy)};
+  const int zs[2] = {mirror_single_i(z0, v.sz), mirror_single_i(z0 + 1, v.sz)};
+  float val[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    val[c] = __ldg(v.img + ((Off)zs[(c >> 2) & 1] * v.sy + ys[(c >> 1) & 1]) * v.sx + xs[c & 1]);
+  return corner_sum(val, tx - fx0, ty - fy0, tz - fz0);
 }
 
 // The reference normalises in double (and multiplies blending weights by a double table);
@@ -140,8 +136,8 @@ __device__ __forceinline__ FF ff_mul(FF a, FF b) {
 }
 
 // BlendingRealRandomAccess.computeWeight (:91-121) on the view interval [0, size)
-__device__ __forceinline__ float blend_weight(float lx, float ly, float lz, int sx, int sy, int sz, float3 border,
-                                              float3 range) {
+__device__ __noinline__ float blend_weight(float lx, float ly, float lz, int sx, int sy, int sz, float3 border,
+                                           float3 range) {
   const float loc[3] = {lx, ly, lz};
   const float dm1[3] = {(float)(sx - 1), (float)(sy - 1), (float)(sz - 1)};
   const float b[3] = {border.x, border.y, border.z};
@@ -150,7 +146,6 @@ __device__ __forceinline__ float blend_weight(float lx, float ly, float lz, int 
 #pragma unroll
   for (int d = 0; d < 3; ++d) dist3[d] = fmaxf(0.f, fminf(loc[d] - b[d], dm1[d] - loc[d] - b[d]));
   if (dist3[0] == 0.f || dist3[1] == 0.f || dist3[2] == 0.f) return 0.f;
-  if (dist3[0] >= r[0] && dist3[1] >= r[1] && dist3[2] >= r[2]) return 1.f;  // beyond every blending zone
   float w = 1.f;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
@@ -185,58 +180,108 @@ __device__ __forceinline__ float blend_weight(float lx, float ly, float lz, int 
   return w;
 }
 
-// Output voxel (x, y, z): the resampled view (0 outside it) and its blending weight.
-template <class Index>
-__device__ __forceinline__ void transform_voxel(const float* __restrict__ view, int sx, int sy, int sz,
-                                                const Affine& inv, float s0, float s1, float s2, bool want_img,
-                                                bool want_blend, float3 border, float3 range, float& v, float& wgt) {
-  const float t0 = inv.m[0] * s0 + inv.m[1] * s1 + inv.m[2] * s2 + inv.m[3];
-  const float t1 = inv.m[4] * s0 + inv.m[5] * s1 + inv.m[6] * s2 + inv.m[7];
-  const float t2 = inv.m[8] * s0 + inv.m[9] * s1 + inv.m[10] * s2 + inv.m[11];
+// Blending: border and range per axis, and a box of positions whose weight is 1 (beyond every
+// blending zone), a rounding's width inside the exact one.
+struct Blending {
+  float3 border, range;
+  float lo[3], hi[3];
+};
+
+// One output voxel at view position (t0, t1, t2): the resampled view (0 outside it) and its blending
+// weight.  Nearly every voxel has its eight corners inside the view, and half of them lie beyond the
+// blending zones: they take neither of the calls.  The kernels are bound by instruction issue: 204 ->
+// 170 per voxel and warp at 4 views of 256x256x192 with the corners at fixed offsets from one 32-bit
+// address and a plain box for a weight of 1 (80 -> 70 us a view along x, 71 unchanged along z, where a
+// thread's four voxels share no terms of their positions); the image alone takes 112, a weight alone 113.
+template <class Off>
+__device__ __forceinline__ void transform_voxel(const View& view, float t0, float t1, float t2, bool want_img,
+                                                bool want_blend, const Blending& bl, float& v, float& wgt) {
   v = 0.f;  // no image data (MVDeconvolution.computeQuotient reads 0 as "no data")
-  if (want_img && t0 >= 0.f && t1 >= 0.f && t2 >= 0.f && t0 < (float)sx && t1 < (float)sy && t2 < (float)sz)
-    v = fmaxf(1e-4f, trilinear_mirror<Index>(view, sx, sy, sz, t0, t1, t2));
+  if (want_img && t0 >= 0.f && t1 >= 0.f && t2 >= 0.f) {
+    const float f0 = floorf(t0), f1 = floorf(t1), f2 = floorf(t2);
+    const int x0 = (int)f0, y0 = (int)f1, z0 = (int)f2;
+    if (x0 < view.sx - 1 && y0 < view.sy - 1 && z0 < view.sz - 1) {
+      const Off o = (((Off)z0 * view.sy + y0) * view.sx + x0) * 4;
+      const char* p = reinterpret_cast<const char*>(view.img);
+      const size_t row = (size_t)view.sx * 4, plane = row * view.sy;
+      auto at = [o](const char* base) { return reinterpret_cast<const float*>(base + o); };
+      const float* q[4] = {at(p), at(p + row), at(p + plane), at(p + plane + row)};
+      float val[8];
+#pragma unroll
+      for (int c = 0; c < 8; ++c) val[c] = __ldg(q[c >> 1] + (c & 1));
+      v = fmaxf(1e-4f, corner_sum(val, t0 - f0, t1 - f1, t2 - f2));
+    } else if (t0 < (float)view.sx && t1 < (float)view.sy && t2 < (float)view.sz) {
+      v = fmaxf(1e-4f, trilinear_mirror<Off>(view, t0, t1, t2));
+    }
+  }
   // the blending weight is defined everywhere (the border can be negative)
-  wgt = want_blend ? blend_weight(t0, t1, t2, sx, sy, sz, border, range) : 0.f;
+  if (!want_blend)
+    wgt = 0.f;
+  else if (t0 >= bl.lo[0] && t0 <= bl.hi[0] && t1 >= bl.lo[1] && t1 <= bl.hi[1] && t2 >= bl.lo[2] && t2 <= bl.hi[2])
+    wgt = 1.f;
+  else
+    wgt = blend_weight(t0, t1, t2, view.sx, view.sy, view.sz, bl.border, bl.range);
 }
 
-// One thread per output voxel; a block covers a 32 x 8 patch of one z plane, so a warp runs
-// along output x.  For views whose x axis lies closer to output x than to output z.
-template <class Index>
-__global__ void __launch_bounds__(256) transform_view_kernel(const float* __restrict__ view, int sx, int sy, int sz,
-                                                             Affine inv, int ox, int oy, int oz, int nx, int ny,
-                                                             float* __restrict__ out_img,
-                                                             float* __restrict__ out_blend, float3 border,
-                                                             float3 range) {
-  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, z = blockIdx.z;
+// Row d of the inverse at (s0, s1, s2): m0 s0 + m1 s1 (one FMA), + m2 s2 (another), + m3.  The first
+// is the same for voxels that differ in s2 only.
+__device__ __forceinline__ float pos_xy(const Affine& inv, int d, float s0, float s1) {
+  return __fmaf_rn(inv.m[4 * d], s0, __fmul_rn(inv.m[4 * d + 1], s1));
+}
+__device__ __forceinline__ float pos_z(const Affine& inv, int d, float xy, float s2) {
+  return __fadd_rn(__fmaf_rn(inv.m[4 * d + 2], s2, xy), inv.m[4 * d + 3]);
+}
+
+// A thread takes kZRun voxels of consecutive z planes; a block covers a 32 x 8 patch of them, so a
+// warp runs along output x.  For views whose x axis lies closer to output x than to output z.
+constexpr int kZRun = 4;
+template <class Off>
+__global__ void __launch_bounds__(256) transform_view_kernel(const View view, const __grid_constant__ Affine inv, int ox,
+                                                             int oy, int oz, int nx, int ny, int nz,
+                                                             float* __restrict__ out_img, float* __restrict__ out_blend,
+                                                             const __grid_constant__ Blending bl) {
+  const int x = blockIdx.x * 32 + threadIdx.x, y = blockIdx.y * 8 + threadIdx.y, z0 = blockIdx.z * kZRun;
   if (x >= nx || y >= ny) return;
-  const long long i = ((long long)z * ny + y) * nx + x;
-  float v, wgt;
-  transform_voxel<Index>(view, sx, sy, sz, inv, (float)(x + ox), (float)(y + oy), (float)(z + oz), out_img != nullptr,
-                         out_blend != nullptr, border, range, v, wgt);
-  if (out_img) out_img[i] = v;
-  if (out_blend) out_blend[i] = wgt;
+  const long long plane = (long long)ny * nx;
+  long long i = z0 * plane + (long long)y * nx + x;
+  const float s0 = (float)(x + ox), s1 = (float)(y + oy);
+  const float a0 = pos_xy(inv, 0, s0, s1), a1 = pos_xy(inv, 1, s0, s1), a2 = pos_xy(inv, 2, s0, s1);
+#pragma unroll
+  for (int k = 0; k < kZRun; ++k, i += plane) {
+    if (z0 + k >= nz) break;
+    const float s2 = (float)(z0 + k + oz);
+    float v, wgt;
+    transform_voxel<Off>(view, pos_z(inv, 0, a0, s2), pos_z(inv, 1, a1, s2), pos_z(inv, 2, a2, s2), out_img != nullptr,
+                         out_blend != nullptr, bl, v, wgt);
+    if (out_img) out_img[i] = v;
+    if (out_blend) out_blend[i] = wgt;
+  }
 }
 
 // The same for views whose x axis lies closer to output z (a rotation near 90 degrees about
 // y): a block covers 32 z x 32 x of one y row and a warp runs along output z, so its lanes
 // read neighbouring voxels of one view row instead of 32 view planes.  The results are staged
 // in shared memory (rows padded to 33: conflict-free both ways) and stored along x.
-template <class Index>
-__global__ void __launch_bounds__(256) transform_view_zfast_kernel(
-    const float* __restrict__ view, int sx, int sy, int sz, Affine inv, int ox, int oy, int oz, int nx, int ny,
-    int nz, float* __restrict__ out_img, float* __restrict__ out_blend, float3 border, float3 range) {
+template <class Off>
+__global__ void __launch_bounds__(256) transform_view_zfast_kernel(const View view, const __grid_constant__ Affine inv,
+                                                                   int ox, int oy, int oz, int nx, int ny, int nz,
+                                                                   float* __restrict__ out_img,
+                                                                   float* __restrict__ out_blend,
+                                                                   const __grid_constant__ Blending bl) {
   __shared__ float s_img[32][33], s_w[32][33];  // [z][x] within the tile
   const int lane = threadIdx.x, warp = threadIdx.y;
   const int x0 = blockIdx.x * 32, y = blockIdx.y, z0 = blockIdx.z * 32;
   const int z = z0 + lane;
+  const float s1 = (float)(y + oy), s2 = (float)(z + oz);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     const int xl = warp + 8 * k, x = x0 + xl;
     if (x < nx && z < nz) {
+      const float s0 = (float)(x + ox);
       float v, wgt;
-      transform_voxel<Index>(view, sx, sy, sz, inv, (float)(x + ox), (float)(y + oy), (float)(z + oz),
-                             out_img != nullptr, out_blend != nullptr, border, range, v, wgt);
+      transform_voxel<Off>(view, pos_z(inv, 0, pos_xy(inv, 0, s0, s1), s2), pos_z(inv, 1, pos_xy(inv, 1, s0, s1), s2),
+                           pos_z(inv, 2, pos_xy(inv, 2, s0, s1), s2), out_img != nullptr, out_blend != nullptr, bl, v,
+                           wgt);
       s_img[lane][xl] = v;
       s_w[lane][xl] = wgt;
     }
@@ -361,7 +406,8 @@ __device__ __forceinline__ bool exact_view_sum(const float* wv, int nv, float& h
 // two-sums hold it when their own sum is exact.  A quarter of the instructions of the integer sum,
 // which takes what is left (false): smaller, larger, negative or non-finite weights.  Blending
 // weights lie in this range but for the last thousandths of a zone.  With the shared reciprocal it
-// takes the kernel from 236 to 123 us at 4 views of 256x256x192 (403 MB: 1.7 -> 3.3 TB/s).
+// took the kernel from 236 to 123 us at 4 views of 256x256x192 (403 MB), and normalized_weight to 95
+// (4.2 TB/s).
 __device__ __forceinline__ bool float_view_sum(const float* wv, int nv, float& hi, float& lo) {
   bool ok = true;
 #pragma unroll
@@ -378,14 +424,29 @@ __device__ __forceinline__ bool float_view_sum(const float* wv, int nv, float& h
 #pragma unroll
   for (int v = 1; v < 16; ++v)
     if (v < nv) {
-      float e1, e2;
+      float e1, e2 = 0.f;
       s = two_sum(s, wv[v], e1);
-      e = two_sum(e, e1, e2);
+      e = v == 1 ? e1 : two_sum(e, e1, e2);
       exact = exact && e2 == 0.f;
     }
   hi = __fadd_rn(s, e);
   lo = __fsub_rn(e, __fsub_rn(hi, s));  // |s| >= |e|: exact
   return exact;
+}
+
+// fl(w / norm * osem) for a weight that is 0 or in [2^-24, 2], norm in [1, 32] and osem in [2^-30, 2^30]:
+// ff_quotient, ff_mul and round_pair without their tests for values too small or too large (21 of 50
+// instructions a view).  At a power of two only an exact result is certain (the half ulp below is smaller).
+__device__ __forceinline__ bool normalized_weight(float w, float norm, float rcp, FF os, float& y) {
+  const float q = __fmul_rn(w, rcp);
+  const float ql = __fmul_rn(__fmaf_rn(-q, norm, w), rcp);
+  const float p = __fmul_rn(q, os.hi);
+  const float pl = __fadd_rn(__fmaf_rn(q, os.hi, -p), __fmaf_rn(ql, os.hi, __fmul_rn(q, os.lo)));
+  y = __fadd_rn(p, pl);
+  const float d = __fadd_rn(__fsub_rn(p, y), pl);
+  const unsigned b = __float_as_uint(y);
+  const float limit = __fmul_rn(__uint_as_float(b & 0x7f800000u), 0x1p-24f * 0.99993896484375f);
+  return fabsf(d) <= limit && ((b & 0x007fffffu) != 0u || d == 0.f);
 }
 
 struct Deferred {  // voxels left to the double pass
@@ -402,6 +463,55 @@ struct Deferred {  // voxels left to the double pass
 // (float)(w_v / sum_w) with no guard on the sum (0 / 0 gives NaN where no view has weight, as
 // in the reference), then min(1, w * (float)osem) in float.
 // osem arrives as a float pair too (osem_hi + osem_lo == osem to ~48 bits).
+// The general way: any weight, any OSEM factor, both modes.  plain: s_hi + s_lo holds the sum already.
+// false when a rounding is not certain.
+template <int NV>
+__device__ __forceinline__ bool normalize_voxel_pairs(const float* wv, bool plain, float s_hi, float s_lo, FF os,
+                                                      bool unit, int mode, float* out) {
+  constexpr int nv = NV;
+  if (!plain && !exact_view_sum(wv, nv, s_hi, s_lo)) {
+    double sum_d = 0.0;
+#pragma unroll
+    for (int v = 0; v < 16; ++v)
+      if (v < nv) sum_d += (double)wv[v];
+    s_hi = (float)sum_d;
+    s_lo = (float)(sum_d - (double)s_hi);
+  }
+  bool certain = fabsf(s_hi) < 1.26765060022822940e30f;  // 2^100: reciprocals stay normal
+  if (mode == 0) {
+    // sum_w > 1 ? (float)sum_w : 1, NaN included (a NaN sum gives 1)
+    const float norm = fmaxf(s_hi, 1.f);
+    const float rcp = __frcp_rn(norm);
+#pragma unroll
+    for (int v = 0; v < 16; ++v)
+      if (v < nv) {
+        float y;
+        if (unit) {
+          y = __fdiv_rn(wv[v], norm);
+        } else {
+          const FF q = ff_quotient(wv[v], FF{norm, 0.f}, rcp);
+          certain = !tiny(wv[v]) && !tiny(q.hi) && round_pair(ff_mul(q, os), y) && certain;
+        }
+        out[v] = java_min1(y);
+      }
+  } else {
+    const FF sum = {s_hi, s_lo};
+    const float rcp = __frcp_rn(s_hi);
+#pragma unroll
+    for (int v = 0; v < 16; ++v)
+      if (v < nv) {
+        float x = 0.f;
+        if (s_hi == 0.f) {  // a sum of floats is 0 or at least 2^-149 in magnitude
+          x = __fdiv_rn(wv[v], 0.f);  // w / 0: NaN (0 / 0) or an infinity, as in double
+        } else {
+          certain = !tiny(wv[v]) && !tiny(s_hi) && round_pair(ff_quotient(wv[v], sum, rcp), x) && certain;
+        }
+        out[v] = java_min1(__fmul_rn(x, os.hi));  // (float)osemspeedup: the float osem
+      }
+  }
+  return certain;
+}
+
 // The view count is a template parameter: guards on a runtime count would still issue the
 // instructions of all 16 view slots.
 template <int NV>
@@ -410,51 +520,28 @@ __global__ void normalize_weights_kernel(WeightPtrs w, long long n, double osem,
   constexpr int nv = NV;
   const FF os = {osem_hi, osem_lo};
   const bool unit = osem == 1.0;
+  // the common call: VIRTUAL weights with a factor
+  const bool short_way = mode == 0 && !unit && fabsf(osem_hi) >= 0x1p-30f && fabsf(osem_hi) <= 0x1p30f;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     float wv[16], out[16];
 #pragma unroll
     for (int v = 0; v < 16; ++v)
       if (v < nv) wv[v] = w.p[v][i];
     float s_hi, s_lo;  // (float)sum_w and (float)(sum_w - s_hi)
-    if (!float_view_sum(wv, nv, s_hi, s_lo) && !exact_view_sum(wv, nv, s_hi, s_lo)) {
-      double sum_d = 0.0;
-#pragma unroll
-      for (int v = 0; v < 16; ++v)
-        if (v < nv) sum_d += (double)wv[v];
-      s_hi = (float)sum_d;
-      s_lo = (float)(sum_d - (double)s_hi);
-    }
-    bool certain = fabsf(s_hi) < 1.26765060022822940e30f;  // 2^100: reciprocals stay normal
-    if (mode == 0) {
-      // sum_w > 1 ? (float)sum_w : 1, NaN included (a NaN sum gives 1)
+    const bool plain = float_view_sum(wv, nv, s_hi, s_lo);
+    bool certain = true;
+    if (plain && short_way) {
       const float norm = fmaxf(s_hi, 1.f);
       const float rcp = __frcp_rn(norm);
 #pragma unroll
       for (int v = 0; v < 16; ++v)
         if (v < nv) {
           float y;
-          if (unit) {
-            y = __fdiv_rn(wv[v], norm);
-          } else {
-            const FF q = ff_quotient(wv[v], FF{norm, 0.f}, rcp);
-            certain = !tiny(wv[v]) && !tiny(q.hi) && round_pair(ff_mul(q, os), y) && certain;
-          }
-          out[v] = java_min1(y);
+          certain = normalized_weight(wv[v], norm, rcp, os, y) && certain;
+          out[v] = fminf(1.f, y);
         }
     } else {
-      const FF sum = {s_hi, s_lo};
-      const float rcp = __frcp_rn(s_hi);
-#pragma unroll
-      for (int v = 0; v < 16; ++v)
-        if (v < nv) {
-          float x = 0.f;
-          if (s_hi == 0.f) {  // a sum of floats is 0 or at least 2^-149 in magnitude
-            x = __fdiv_rn(wv[v], 0.f);  // w / 0: NaN (0 / 0) or an infinity, as in double
-          } else {
-            certain = !tiny(wv[v]) && !tiny(s_hi) && round_pair(ff_quotient(wv[v], sum, rcp), x) && certain;
-          }
-          out[v] = java_min1(__fmul_rn(x, osem_hi));  // (float)osemspeedup: the float osem
-        }
+      certain = normalize_voxel_pairs<NV>(wv, plain, s_hi, s_lo, os, unit, mode, out);
     }
     if (certain) {
 #pragma unroll
@@ -662,26 +749,37 @@ extern "C" int mvd_transform_view(const float* view, const int* vd, const double
     }
     MVD_CHECK(cudaSetDevice(devCUDA));
     upload_lut(devCUDA);
-    const float3 b = out_blend ? make_float3(border[0], border[1], border[2]) : make_float3(0.f, 0.f, 0.f);
-    const float3 r = out_blend ? make_float3(blending[0], blending[1], blending[2]) : make_float3(1.f, 1.f, 1.f);
+    Blending bl{};
+    if (out_blend) {
+      bl.border = make_float3(border[0], border[1], border[2]);
+      bl.range = make_float3(blending[0], blending[1], blending[2]);
+      for (int d = 0; d < 3; ++d) {
+        // l >= border + range and size - 1 - l >= border + range, each moved in by more than the
+        // roundings of the weight's own differences (2^-23 of the largest of them)
+        const double margin = 1e-6 * (std::fabs(border[d]) + std::fabs(blending[d]) + vd[d] + 1.0);
+        const double inner = (double)border[d] + blending[d] + margin;
+        bl.lo[d] = (float)inner;
+        bl.hi[d] = (float)((double)(vd[d] - 1) - inner);
+      }
+    }
     if (od[2] > 65535 || od[1] > 8 * 65535) {
       set_last_error("output height above 524280 or depth above 65535");
       return MVD_ERR_ARG;
     }
-    const bool narrow = (long long)vd[0] * vd[1] * vd[2] < (1LL << 31);
+    const bool narrow = (long long)vd[0] * vd[1] * vd[2] < (1LL << 30);
+    const View v{view, vd[0], vd[1], vd[2]};
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     // the warp runs along the output axis that moves the view position most along view x
     // (inv.m[0] and inv.m[2]: d(view x) / d(output x) and d(view x) / d(output z))
     if (std::fabs(inv.m[2]) > std::fabs(inv.m[0]) && od[1] <= 65535) {
       const dim3 grid((od[0] + 31) / 32, od[1], (od[2] + 31) / 32);
-      (narrow ? transform_view_zfast_kernel<int> : transform_view_zfast_kernel<long long>)<<<grid, dim3(32, 8), 0,
-                                                                                              s>>>(
-          view, vd[0], vd[1], vd[2], inv, offset[0], offset[1], offset[2], od[0], od[1], od[2], out_img, out_blend, b,
-          r);
+      (narrow ? transform_view_zfast_kernel<unsigned> : transform_view_zfast_kernel<long long>)<<<grid, dim3(32, 8), 0,
+                                                                                                   s>>>(
+          v, inv, offset[0], offset[1], offset[2], od[0], od[1], od[2], out_img, out_blend, bl);
     } else {
-      const dim3 grid((od[0] + 31) / 32, (od[1] + 7) / 8, od[2]);
-      (narrow ? transform_view_kernel<int> : transform_view_kernel<long long>)<<<grid, dim3(32, 8), 0, s>>>(
-          view, vd[0], vd[1], vd[2], inv, offset[0], offset[1], offset[2], od[0], od[1], out_img, out_blend, b, r);
+      const dim3 grid((od[0] + 31) / 32, (od[1] + 7) / 8, (od[2] + kZRun - 1) / kZRun);
+      (narrow ? transform_view_kernel<unsigned> : transform_view_kernel<long long>)<<<grid, dim3(32, 8), 0, s>>>(
+          v, inv, offset[0], offset[1], offset[2], od[0], od[1], od[2], out_img, out_blend, bl);
     }
     MVD_CHECK(cudaGetLastError());
     count_launch();

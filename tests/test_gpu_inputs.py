@@ -223,6 +223,20 @@ def test_normalize_weights_at_the_edges_of_the_float_sum(mode, views):
             np.testing.assert_array_equal(d.cpu().numpy(), w)
 
 
+@pytest.mark.parametrize("blend", [(12.0, 9.0, 4.0), (0.25, 5.0, 3.0), (30.0, 2.5, 60.0)])
+@pytest.mark.parametrize("border", [(0.0, 0.0, 0.0), (-3.25, 2.5, -1.0)])
+def test_blending_weight_at_the_edges_of_the_inner_box(border, blend):
+    """Weights around the positions where they become 1 (a range below a voxel and one wider than the view
+    included), bit-equal under the identity registration, over depths that are no multiple of a
+    thread's run of planes."""
+    torch = pytest.importorskip("torch")
+    lib = native.load()
+    view, out, offset = (21, 33, 47), (27, 39, 53), (-3, -3, -3)
+    eye = [1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0]
+    got = _blend_on_device(lib, torch, view, out, border, blend, offset)
+    np.testing.assert_array_equal(got, O.transform_weights(view, eye, offset, out, border, blend))
+
+
 @pytest.mark.parametrize("n", [1, 3, 127, 129, 40001])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_weight_overlap_of_slices(n, shift):
