@@ -82,3 +82,17 @@ def test_set_kernel_changes_the_model(case):
     assert d.forward() == pytest.approx(O.poisson_nll(psi, p.views, p.weights, k), rel=2e-5)
     d.set_kernel(0, 1, old)
     assert d.forward() == pytest.approx(base, rel=1e-6)
+
+
+@pytest.mark.parametrize("shape,psf", [((40, 11, 9), (11, 15, 17)),   # two positions per voxel and axis
+                                       ((7, 34, 5), (19, 5, 17))])    # more than two along x and z
+def test_fold_of_wide_kernels_matches_oracle_gradient(shape, psf):
+    """The mirror extension reaches across the volume: voxels gather several positions on every axis
+    (tolerance as above)."""
+    p = S.make_problem(5, shape_xyz=shape, psf_size_xyz=psf, n_blobs=10, n_views=2, iterations=1)
+    with Deconvolution(p.views, p.weights, p.psfs, p.psftype, p.lam) as d:
+        d.run(1)
+        psi = d.get_psi().astype(np.float64)
+        k1 = [d.kernel(v, 1).astype(np.float64) for v in range(2)]
+        g_psi, _ = d.backward()
+    assert rel_l2(g_psi, O.poisson_nll_grad(psi, p.views, p.weights, k1)[0]) < 1e-4
