@@ -27,9 +27,9 @@
 // forward pass) instead of overlapping.  Larger tiles win although they leave one CTA per SM: the
 // halo they save is worth more than the second CTA's overlap (512x512x256, 31x31x61 PSFs: 7.70 ms
 // per iteration at up to 226 KB per plane against 8.98 at 112 KB and 9.76 at 74 KB).
-// Measured per iteration, scalar kernels / these: 4 views of 512x512x256 9.17 / 7.70 ms; 4 views of
-// 256x256x192 with 15x15x41 PSFs 1.70 / 1.64 ms; 6 crops of 256^3 2.10 / 1.61 ms (shapes without
-// compiled scalar kernels); 2 views of 128x128x64 0.16 / 0.13 ms.
+// Measured per iteration, scalar kernels / these: 4 views of 512x512x256 9.17 / 7.51 ms; 4 views of
+// 256x256x192 with 15x15x41 PSFs 1.70 / 1.54 ms; 6 crops of 256^3 2.10 / 1.46 ms (shapes without
+// compiled scalar kernels); 2 views of 128x128x64 0.16 / 0.11 ms.
 #pragma once
 #include "kernels.cuh"
 #include "pair_fft.cuh"
