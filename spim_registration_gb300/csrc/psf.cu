@@ -7,6 +7,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cfloat>
 #include <climits>
 #include <cmath>
 #include <string>
@@ -63,6 +64,14 @@ __device__ __forceinline__ int wrap(int i, int n) {  // i >= 0; one subtraction 
 constexpr int kRunY = 4, kRunZ = 8;  // PSF voxels of a thread: 4 x 8 at one x, lanes along x
 constexpr int kExtractThreads = 128;
 
+// (1 - a) v0 + a v1 with one rounding beside that of v1 - v0, which is exact for whole numbers and near
+// neighbours; the weighted form (three roundings) only where an infinity or NaN comes out, for its
+// result there.
+__device__ __forceinline__ float lerp(float a, float v0, float v1) {
+  const float t = __fmaf_rn(a, v1 - v0, v0);
+  return fabsf(t) <= FLT_MAX ? t : __fmaf_rn(a, v1, (1.f - a) * v0);
+}
+
 // Partial sums of the beads [chunk * per, chunk * per + per): part[chunk][voxel].  The trilinear
 // weights of a bead are the same for every voxel, so a thread interpolates a 5 x 9 patch of rows
 // along x once and then along y and z: 2.8 loads and 7 multiply-adds per voxel and bead.  One
@@ -95,12 +104,12 @@ __global__ void __launch_bounds__(kExtractThreads, 4) extract_partial_kernel(
 #pragma unroll
       for (int y = 0; y <= kRunY; ++y) {
         const float* r = slice + (long long)row[y] * sx;
-        t[y] = __fmaf_rn(b.ax, __ldg(r + x1), (1.f - b.ax) * __ldg(r + x0));
+        t[y] = lerp(b.ax, __ldg(r + x0), __ldg(r + x1));
       }
 #pragma unroll
       for (int y = 0; y < kRunY; ++y) {
-        const float u = __fmaf_rn(b.ay, t[y + 1], (1.f - b.ay) * t[y]);
-        if (k > 0) acc[k - 1][y] += __fmaf_rn(b.az, u, (1.f - b.az) * last[y]);
+        const float u = lerp(b.ay, t[y], t[y + 1]);
+        if (k > 0) acc[k - 1][y] += lerp(b.az, last[y], u);
         last[y] = u;
       }
     }
@@ -114,15 +123,21 @@ __global__ void __launch_bounds__(kExtractThreads, 4) extract_partial_kernel(
       if (y0 + y < py && z0 + k < pz) out[((long long)(z0 + k) * py + y0 + y) * px] = acc[k][y];
 }
 
-// psf = the sum of the partial sums in their order; the extremes of each block's voxels
+// psf = the sum of the partial sums in their order, with the additions' own errors (two-sums) added at
+// the end; the extremes of each block's voxels
 __global__ void extract_sum_kernel(const float* __restrict__ part, int chunks, int n, float* __restrict__ psf,
                                    float2* __restrict__ ends) {
   __shared__ float2 red[32];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   float lo = INFINITY, hi = -INFINITY;
   if (i < n) {
-    float s = 0.f;
-    for (int c = 0; c < chunks; ++c) s += part[(long long)c * n + i];
+    float s = 0.f, e = 0.f;
+    for (int c = 0; c < chunks; ++c) {
+      const float v = part[(long long)c * n + i], t = s + v, bb = t - s;
+      e += (s - (t - bb)) + (v - bb);
+      s = t;
+    }
+    if (fabsf(s + e) <= FLT_MAX) s += e;
     psf[i] = s;
     lo = fminf(lo, s);
     hi = fmaxf(hi, s);
