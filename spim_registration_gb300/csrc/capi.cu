@@ -1391,18 +1391,21 @@ extern "C" int mvd_backward(mvd_decon* h, float* grad_psi, float* const* grad_ps
   cudaStream_t s = h->stream;
   MVD_CHECK(cudaMemsetAsync(h->g_psi.p, 0, h->N * sizeof(float), s));
   MVD_CHECK(cudaMemsetAsync(h->d_nll.p, 0, sizeof(double), s));
-  MVD_CHECK(cudaMemsetAsync(h->r.p, 0, h->N * sizeof(float), s));  // zero outside the views' data boxes
   for (int v = 0; v < h->V; ++v) {
     const ConvPlan& p = h->adj_plan(v);
     mvd_decon::AdjView& a = h->adj[v];
     const auto& k = h->kd[v];
     // recompute this view's blur and residual (no blurred view is kept between calls)
     enqueue_blur_nll(h, v, true);
-    // dNLL/dpsi: residual (zero outside) convolved with mirror(kernel1) on the extended grid,
-    // then folded back through the mirror-single extension
+    // dNLL/dpsi: residual (zero outside the view's data box: beyond it, h->r still holds an earlier
+    // view's) convolved with mirror(kernel1) on the extended grid, then folded back through the
+    // mirror-single extension
     const ConvPlan& e = *a.ext;
     float2* se = h->spec_ext.as<float2>();
-    launch_fwd_value_tiles(h->pt, e, TileSet::All, h->r.as<float>(), h->dims[0], h->dims[1], h->dims[2], 0.f, se, s);
+    const GatherValue residual =
+        GatherValue::box(h->r.as<float>(), h->dims[0], h->dims[1], h->dims[2], 0.f, p.box_lo[0], p.box_lo[1],
+                         p.box_lo[2], p.box_hi[0], p.box_hi[1], p.box_hi[2]);
+    launch_fwd_value_tiles(h->pt, e, TileSet::All, residual, se, s);
     launch_z(h->pt, e, se, a.otf_m.as<float2>(), s);
     const long long off = ((long long)(k[2] / 2) * e.ny + k[1] / 2) * e.nx + k[0] / 2;
     launch_inv_store_tiles(h->pt, e, TileSet::All, se, h->c_ext.as<float>() + off, e.nx, e.ny, s);

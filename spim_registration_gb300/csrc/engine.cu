@@ -930,7 +930,7 @@ void build_otf(PlanTable& pt, const ConvPlan& plan, const float* kernel, float2*
   count_launch();
   // one tile covering the placed kernel volume exactly; its spectrum goes to `otf`.  The product of
   // two spectra carries the passes' scale twice.
-  launch_fwd_value_tiles(pt, plan, TileSet::Full, scratch.as<float>(), tx, ty, tz, 0.f, otf, s);
+  launch_fwd_value_tiles(pt, plan, TileSet::Full, GatherValue::full(scratch.as<float>(), tx, ty, tz, 0.f), otf, s);
   const double sc = spectrum_scale(plan) * spectrum_scale(plan);
   launch_z_forward(pt, plan, TileSet::Full, otf, (float)(1.0 / (sc * tx * ty * tz)), s);
 }

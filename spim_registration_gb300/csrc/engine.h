@@ -263,10 +263,10 @@ inline void launch_after(void (*k)(P...), int grid, int threads, size_t smem, cu
   MVD_CHECK(cudaLaunchKernelEx(&c, k, static_cast<P>(args)...));
 }
 
-// Forward plane pass gathering from a (vx, vy, vz) volume with a constant border value; and the
+// Forward plane pass gathering from a volume's box with a constant value outside it; and the
 // forward-only, scaled z pass (kernel spectra; spectra of the PSF gradient).
-void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float* vol, int vx, int vy, int vz,
-                            float value, float2* spec, cudaStream_t s);
+void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const GatherValue& g, float2* spec,
+                            cudaStream_t s);
 void launch_z_forward(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, float scale, cudaStream_t s);
 
 // The three passes, for fused use by the deconvolution handle.

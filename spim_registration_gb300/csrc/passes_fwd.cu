@@ -143,9 +143,8 @@ void launch_fwd_value(PlanTable& pt, const ConvPlan& p, const float* vol, float 
                   p.threads_plane, p.ax.T, p.ay.T, spec, g, s, p.generic, p.staged);
 }
 
-void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float* vol, int vx, int vy, int vz,
-                            float value, float2* spec, cudaStream_t s) {
-  GatherValue g = GatherValue::full(vol, vx, vy, vz, value);
+void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const GatherValue& g, float2* spec,
+                            cudaStream_t s) {
   if (p.paired) return pair_fwd_value(p, set, g, spec, s);
   const bool all = set == TileSet::All;
   launch_fwd_impl(pt, (all ? p.d_tiles : p.d_otf_tile).as<TileDesc>(), (all ? p.d_items_fwd : p.d_otf_fwd).as<int2>(),

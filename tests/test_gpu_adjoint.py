@@ -96,3 +96,24 @@ def test_fold_of_wide_kernels_matches_oracle_gradient(shape, psf):
         k1 = [d.kernel(v, 1).astype(np.float64) for v in range(2)]
         g_psi, _ = d.backward()
     assert rel_l2(g_psi, O.poisson_nll_grad(psi, p.views, p.weights, k1)[0]) < 1e-4
+
+
+def test_backward_of_views_cropped_to_different_boxes():
+    """Each view's residual counts inside its own data box only, also where another view's box
+    reaches further (tolerance as above)."""
+    p = S.make_problem(5, shape_xyz=(36, 32, 28), psf_size_xyz=(7, 7, 11), n_blobs=40, n_views=3, iterations=1)
+    boxes = [((0, 0, 0), (20, 32, 28)), ((12, 3, 5), (36, 30, 23)), ((0, 16, 0), (31, 32, 17))]  # x, y, z
+    for v, (lo, hi) in enumerate(boxes):
+        for a in (p.views[v], p.weights[v]):
+            keep = a[lo[2]:hi[2], lo[1]:hi[1], lo[0]:hi[0]].copy()
+            a[...] = 0
+            a[lo[2]:hi[2], lo[1]:hi[1], lo[0]:hi[0]] = keep
+    with Deconvolution(p.views, p.weights, p.psfs, p.psftype, p.lam) as d:
+        d.run(1)
+        psi = d.get_psi().astype(np.float64)
+        k1 = [d.kernel(v, 1).astype(np.float64) for v in range(3)]
+        g_psi, g_psf = d.backward()
+    w_psi, w_psf = O.poisson_nll_grad(psi, p.views, p.weights, k1)
+    assert rel_l2(g_psi, w_psi) < 1e-4
+    for a, b in zip(g_psf, w_psf):
+        assert rel_l2(a, b) < 1e-4
