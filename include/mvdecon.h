@@ -230,7 +230,9 @@ int mvd_weight_overlap(const float* const* weights, int num_views, long long n, 
  * locations (x, y, z triples, doubles, in the view's pixel frame; host array) of the view
  * (device, dims_xyz) interpolated trilinearly, extended periodically, at p - psf_dims / 2 +
  * location; locations are added in the given order.  normalize != 0 then applies
- * ExtractPSF.normalize (:298-316): (v - min) / (max - min).  psf: device, overwritten. */
+ * ExtractPSF.normalize (:298-316): (v - min) / (max - min).  psf: device, overwritten.
+ * A pageable locations array has been read when the call returns, a page-locked one when the stream
+ * has passed the call.  A call on a stream under capture reads the array again at every replay. */
 int mvd_extract_psf(const float* img, const int* dims_xyz, const double* locations_xyz, int num_locations,
                     const int* psf_dims_xyz, float* psf, int normalize, int devCUDA, void* stream);
 /* ExtractPSF.transformPSF (:325-372), host only: the odd size of the transformed PSF (the

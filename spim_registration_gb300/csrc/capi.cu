@@ -195,17 +195,6 @@ struct WaitOnError {
   }
 };
 
-// whether copying from p returns before the copy is done (device memory, or host memory
-// that is page-locked); a copy from pageable host memory holds the calling thread
-bool async_copy_source(const void* p) {
-  cudaPointerAttributes a{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged || a.type == cudaMemoryTypeHost;
-}
-
 std::mutex g_ctx_mu;
 std::unordered_map<int, std::unique_ptr<DeviceCtx>> g_ctx;
 

@@ -43,6 +43,15 @@ void upload_table(void* dst, const void* src, size_t bytes) {
     MVD_CHECK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
 }
 
+bool async_copy_source(const void* p) {
+  cudaPointerAttributes a{};
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged || a.type == cudaMemoryTypeHost;
+}
+
 void keep_pool_memory(int dev) {
   static std::mutex mu;
   static std::vector<bool> done;

@@ -68,6 +68,10 @@ class AllocScope {
 };
 cudaStream_t alloc_stream();
 void upload_table(void* dst, const void* src, size_t bytes);
+// Whether p is device memory, or host memory that CUDA knows (page-locked, managed): a copy from it
+// returns before it is done.  A copy from pageable host memory mostly holds the calling thread, but
+// need not.
+bool async_copy_source(const void* p);
 // Keep freed pool memory cached in this process instead of returning it at every
 // synchronisation (the device's default pool; a process-local attribute).
 void keep_pool_memory(int dev);

@@ -11,7 +11,6 @@
 #include <climits>
 #include <cmath>
 #include <string>
-#include <vector>
 
 #include "../../include/mvdecon.h"
 #include "engine.h"
@@ -52,6 +51,25 @@ struct Bead {
   int x, y, z;
   float ax, ay, az;
 };
+
+// The beads of n locations (x, y, z triples), split in double (exactly): the device does it from the
+// caller's own array, so that a captured call has no host memory of its own that a replay would read.
+__global__ void split_beads_kernel(const double* __restrict__ locations, int n, int3 dims, int3 half,
+                                   Bead* __restrict__ beads) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l >= n) return;
+  const int size[3] = {dims.x, dims.y, dims.z}, h[3] = {half.x, half.y, half.z};
+  int base[3];
+  float frac[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const double t = locations[3LL * l + d], f = floor(t);
+    frac[d] = (float)(t - f);  // NaN for a location that is not finite
+    const double b = isfinite(t) ? fmod(f - (double)h[d], (double)size[d]) : 0.0;
+    base[d] = (int)(b < 0.0 ? b + size[d] : b);
+  }
+  beads[l] = Bead{base[0], base[1], base[2], frac[0], frac[1], frac[2]};
+}
 
 __device__ __forceinline__ int wrap(int i, int n) {  // i >= 0; one subtraction unless the PSF is larger than the view
   if (i >= n) {
@@ -217,6 +235,23 @@ bool invert(const double* a, Affine64& out) {
 
 int blocks_for(long long n) { return (int)((n + 255) / 256); }
 
+// An event behind a copy from the caller's memory; the call waits for it, on its way out of an error too.
+struct CopyDone {
+  cudaEvent_t e = nullptr;
+  void record(cudaStream_t s) {
+    MVD_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    MVD_CHECK(cudaEventRecord(e, s));
+  }
+  void wait() {
+    if (e) MVD_CHECK(cudaEventSynchronize(e));
+  }
+  ~CopyDone() {
+    if (!e) return;
+    cudaEventSynchronize(e);
+    cudaEventDestroy(e);
+  }
+};
+
 }  // namespace
 
 extern "C" int mvd_transformed_psf_size(const int* psf_dims, const double* model, int* out_dims, double* offset) {
@@ -277,19 +312,6 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
     }
     MVD_CHECK(cudaSetDevice(devCUDA));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    // the beads, with positions split in double (exactly) on the host
-    std::vector<Bead> beads(num_locations);
-    for (int l = 0; l < num_locations; ++l) {
-      int base[3];
-      float frac[3];
-      for (int d = 0; d < 3; ++d) {
-        const double t = locations[3 * l + d], f = std::floor(t);
-        frac[d] = (float)(t - f);  // NaN for a location that is not finite
-        const double b = std::isfinite(t) ? std::fmod(f - (double)(psf_dims[d] / 2), (double)dims[d]) : 0.0;
-        base[d] = (int)(b < 0.0 ? b + dims[d] : b);
-      }
-      beads[l] = Bead{base[0], base[1], base[2], frac[0], frac[1], frac[2]};
-    }
     const int xb = (psf_dims[0] + 31) / 32, yb = (psf_dims[1] + kRunY - 1) / kRunY;
     const long long items_ll = (long long)xb * yb * ((psf_dims[2] + kRunZ - 1) / kRunZ);
     if (items_ll * 32 > INT_MAX) {
@@ -302,13 +324,26 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
     const int per = (int)std::max(1LL, (num_locations + want - 1) / want);
     const int chunks = std::max(1, (num_locations + per - 1) / per);
     const int nends = blocks_for(np);
-    const size_t bb = (beads.size() * sizeof(Bead) + 15) / 16 * 16, eb = (size_t)nends * sizeof(float2);
-    const CallBuf buf(devCUDA, bb + eb + (size_t)chunks * np * sizeof(float), s);
-    Bead* d_beads = buf.as<Bead>();
-    float2* d_ends = reinterpret_cast<float2*>(buf.as<char>() + bb);
-    float* d_part = reinterpret_cast<float*>(buf.as<char>() + bb + eb);
-    if (num_locations > 0)
-      MVD_CHECK(cudaMemcpyAsync(d_beads, beads.data(), beads.size() * sizeof(Bead), cudaMemcpyHostToDevice, s));
+    const size_t lb = (size_t)num_locations * 3 * sizeof(double), bb = ((size_t)num_locations * sizeof(Bead) + 7) / 8 * 8,
+                 eb = (size_t)nends * sizeof(float2);
+    const CallBuf buf(devCUDA, lb + bb + eb + (size_t)chunks * np * sizeof(float), s);
+    double* d_loc = buf.as<double>();
+    Bead* d_beads = reinterpret_cast<Bead*>(buf.as<char>() + lb);
+    float2* d_ends = reinterpret_cast<float2*>(buf.as<char>() + lb + bb);
+    float* d_part = reinterpret_cast<float*>(buf.as<char>() + lb + bb + eb);
+    // nothing of the caller's pageable memory is read once the call has returned
+    CopyDone copied;
+    if (num_locations > 0) {
+      MVD_CHECK(cudaMemcpyAsync(d_loc, locations, lb, cudaMemcpyHostToDevice, s));
+      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+      MVD_CHECK(cudaStreamIsCapturing(s, &capture));
+      if (capture == cudaStreamCaptureStatusNone && !async_copy_source(locations)) copied.record(s);
+      split_beads_kernel<<<(num_locations + 127) / 128, 128, 0, s>>>(
+          d_loc, num_locations, make_int3(dims[0], dims[1], dims[2]),
+          make_int3(psf_dims[0] / 2, psf_dims[1] / 2, psf_dims[2] / 2), d_beads);
+      MVD_CHECK(cudaGetLastError());
+      count_launch();
+    }
     extract_partial_kernel<<<dim3((items * 32 + kExtractThreads - 1) / kExtractThreads, chunks), kExtractThreads, 0, s>>>(
         img, dims[0], dims[1], dims[2], d_beads, num_locations, per, psf_dims[0], psf_dims[1], psf_dims[2], xb, yb, items,
         d_part);
@@ -322,6 +357,7 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
       MVD_CHECK(cudaGetLastError());
       count_launch();
     }
+    copied.wait();
     return MVD_OK;
   } catch (const CudaError& e) {
     set_last_error(e.what());

@@ -2,13 +2,14 @@
 trilinear, summed over the locations), normalisation, the transform into the fused frame and
 ExtractPSF's per-view bookkeeping.  FP32 interpolation: max abs error <= 1e-5 of the output's
 max."""
+import ctypes
 import math
 
 import numpy as np
 import pytest
 
 from oracle import mvdecon_oracle as O
-from spim_registration_gb300 import ExtractPSF
+from spim_registration_gb300 import ExtractPSF, native
 from spim_registration_gb300.psf import extract_psf_local, transform_psf
 
 pytestmark = pytest.mark.gpu
@@ -87,3 +88,54 @@ def test_extraction_runs_and_bead_chunks_match_oracle(shape, psf, beads):
     locs = rng.uniform(-2, 3, (beads, 3)) * np.array(shape[::-1])
     locs[0] = np.round(locs[0])
     _close(extract_psf_local(img, locs, psf), O.extract_psf_local(img, locs, psf))
+
+
+def _extract_on(lib, torch, img, locs_ptr, n, psf, out, stream):
+    native.check(lib.mvd_extract_psf(img.data_ptr(), native.iarr(img.shape[::-1]),
+                                     ctypes.cast(locs_ptr, ctypes.POINTER(ctypes.c_double)), n, native.iarr(psf),
+                                     out.data_ptr(), 0, 0, ctypes.c_void_p(stream.cuda_stream)))
+
+
+def test_captured_extraction_replays_from_the_callers_locations():
+    """A graph captured from the call reads the caller's own (page-locked) array at every replay and
+    no host memory of the call's."""
+    torch = pytest.importorskip("torch")
+    lib = native.load()
+    rng = np.random.default_rng(21)
+    img = (rng.random((30, 32, 34)) * 100).astype(np.float32)
+    first, second = (rng.uniform(0, 30, (40, 3)) for _ in range(2))
+    d_img, locs = torch.from_numpy(img).cuda(), torch.from_numpy(first.copy()).pin_memory()
+    out = torch.empty((11, 7, 9), device="cuda")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    _extract_on(lib, torch, d_img, locs.data_ptr(), 40, (9, 7, 11), out, s)
+    s.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s):
+        _extract_on(lib, torch, d_img, locs.data_ptr(), 40, (9, 7, 11), out, s)
+    for want in (first, second):
+        locs.copy_(torch.from_numpy(want))
+        out.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        _close(out.cpu().numpy(), O.extract_psf_local(img, want, (9, 7, 11)))
+
+
+def test_extraction_is_done_with_pageable_locations_on_return():
+    """The array may be reused as soon as the call returns, with the stream still busy."""
+    torch = pytest.importorskip("torch")
+    lib = native.load()
+    rng = np.random.default_rng(22)
+    d_img = torch.from_numpy((rng.random((30, 32, 34)) * 100).astype(np.float32)).cuda()
+    locs = rng.uniform(0, 30, (200000, 3))
+    outs = [torch.empty((3, 3, 3), device="cuda") for _ in range(2)]
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    for out, busy in zip(outs, (0, 20_000_000)):
+        mine = locs.copy()
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(busy)
+        _extract_on(lib, torch, d_img, mine.ctypes.data, len(mine), (3, 3, 3), out, s)
+        mine[...] = np.nan
+    torch.cuda.synchronize()
+    assert torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
