@@ -191,7 +191,8 @@ int mvd_profile_iteration(mvd_decon* h, double* ms, int* launches);
 int mvd_forward(mvd_decon* h, double* nll);
 int mvd_backward(mvd_decon* h, float* grad_psi, float* const* grad_psf);
 /* Replace kernel1 (the PSF used by the first convolution and the model) or kernel2 of a view,
- * as given (no normalisation), and its spectra -- e.g. after a projected gradient step. */
+ * as given (no normalisation), and its spectra -- e.g. after a projected gradient step.  Waits for
+ * the handle's stream: data may be reused and the spectra are complete when the call returns. */
 int mvd_set_kernel(mvd_decon* h, int view, int which /* 1 or 2 */, const float* data);
 
 /* ----- input preparation (the views in the fused frame and their weights), on the GPU -----

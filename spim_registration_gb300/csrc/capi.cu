@@ -1429,9 +1429,6 @@ extern "C" int mvd_set_kernel(mvd_decon* h, int view, int which, const float* da
   MVD_CHECK(cudaSetDevice(h->dev));
   AllocScope scope(h->stream);
   DevBuf& k = which == 1 ? h->k1[view] : h->k2[view];
-  // copied from pageable memory before the call returns; from page-locked memory by the wait below.
-  // The spectra need no wait: whatever uses them runs on the handle's stream.
-  const bool async_src = async_copy_source(data);
   MVD_CHECK(cudaMemcpyAsync(k.p, data, vox(h->kd[view]) * sizeof(float), cudaMemcpyHostToDevice, h->stream));
   const ConvPlan& p = *h->plans[view];
   build_otf(h->pt, p, k.as<float>(), (which == 1 ? h->otf1[view] : h->otf2[view]).as<float2>(), h->scratch,
@@ -1443,7 +1440,9 @@ extern "C" int mvd_set_kernel(mvd_decon* h, int view, int which, const float* da
     if (a.scalar)
       build_otf(h->pt, *a.scalar, h->k1[view].as<float>(), a.otf1.as<float2>(), h->scratch, h->stream);
   }
-  if (async_src) MVD_CHECK(cudaStreamSynchronize(h->stream));
+  // for the source (CUDA does not promise that a copy from pageable memory has read it by now), and so
+  // that an error of the spectra's kernels is this call's
+  MVD_CHECK(cudaStreamSynchronize(h->stream));
   return MVD_OK;
   MVD_API_END
 }

@@ -117,3 +117,23 @@ def test_backward_of_views_cropped_to_different_boxes():
     assert rel_l2(g_psi, w_psi) < 1e-4
     for a, b in zip(g_psf, w_psf):
         assert rel_l2(a, b) < 1e-4
+
+
+def test_set_kernel_is_complete_on_return():
+    """Whatever the handle's stream still had to do: the kernel's array may be reused, and the spectra
+    are built (an error of theirs is the call's own)."""
+    torch = pytest.importorskip("torch")
+    p = S.make_problem(5, shape_xyz=(96, 96, 96), psf_size_xyz=(61, 61, 61), n_blobs=10, n_views=1, iterations=1)
+    with Deconvolution(p.views, p.weights, p.psfs, p.psftype, p.lam) as d:
+        stream = torch.cuda.ExternalStream(d.stream())
+        rng = np.random.default_rng(3)
+        for _ in range(4):
+            k = rng.random((61, 61, 61), dtype=np.float32)
+            want = k.copy()
+            for _ in range(20):
+                d.run_iteration()
+            d.set_kernel(0, 1, k)
+            idle = stream.query()
+            k[...] = -1.0
+            assert idle
+            np.testing.assert_array_equal(d.kernel(0, 1), want)
