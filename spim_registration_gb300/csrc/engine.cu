@@ -28,17 +28,25 @@ void check_cuda(cudaError_t e, const char* what) {
 }
 
 namespace {
-thread_local cudaStream_t tls_alloc_stream = nullptr;
+thread_local AllocScope* tls_scope = nullptr;
 }
 
-AllocScope::AllocScope(cudaStream_t s) : prev_(tls_alloc_stream) { tls_alloc_stream = s; }
-AllocScope::~AllocScope() { tls_alloc_stream = prev_; }
-cudaStream_t alloc_stream() { return tls_alloc_stream; }
+AllocScope::AllocScope(cudaStream_t s) : stream_(s), prev_(tls_scope) { tls_scope = this; }
+AllocScope::~AllocScope() {
+  tls_scope = prev_;
+  if (!tables_.empty()) cudaStreamSynchronize(stream_);  // idle already but on the way out of an error
+}
+void AllocScope::upload(void* dst, const void* src, size_t bytes) {
+  const char* p = static_cast<const char*>(src);
+  tables_.emplace_back(p, p + bytes);
+  MVD_CHECK(cudaMemcpyAsync(dst, tables_.back().data(), bytes, cudaMemcpyHostToDevice, stream_));
+}
+cudaStream_t alloc_stream() { return tls_scope ? tls_scope->stream() : nullptr; }
 
 void upload_table(void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return;
-  if (tls_alloc_stream)  // pageable source: staged before the call returns
-    MVD_CHECK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, tls_alloc_stream));
+  if (tls_scope)
+    tls_scope->upload(dst, src, bytes);
   else
     MVD_CHECK(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice));
 }
@@ -125,9 +133,9 @@ DevBuf& DevBuf::operator=(DevBuf&& o) noexcept {
 void DevBuf::alloc(size_t b) {
   release();
   if (b == 0) return;
-  if (tls_alloc_stream) {
-    MVD_CHECK(cudaMallocAsync(&p, b, tls_alloc_stream));
-    stream = tls_alloc_stream;
+  if (const cudaStream_t s = alloc_stream()) {
+    MVD_CHECK(cudaMallocAsync(&p, b, s));
+    stream = s;
   } else {
     MVD_CHECK(cudaMalloc(&p, b));
   }

@@ -56,15 +56,21 @@ struct DevBuf {
 
 // Stream-ordered allocation for the DevBufs created on this thread during its lifetime; the
 // stream must outlive them.  Host-to-device uploads of tables go through upload_table(), which is
-// ordered in the same stream (a plain copy could overtake work still using recycled memory).
+// ordered in the same stream (a plain copy could overtake work still using recycled memory).  The
+// scope keeps what is being copied until the stream has read it: a copy from pageable memory need not
+// have done so when it returns, and the tables' own vectors go before that.
 class AllocScope {
  public:
   explicit AllocScope(cudaStream_t s);
   ~AllocScope();
   AllocScope(const AllocScope&) = delete;
   AllocScope& operator=(const AllocScope&) = delete;
+  cudaStream_t stream() const { return stream_; }
+  void upload(void* dst, const void* src, size_t bytes);
  private:
-  cudaStream_t prev_;
+  cudaStream_t stream_;
+  AllocScope* prev_;
+  std::vector<std::vector<char>> tables_;
 };
 cudaStream_t alloc_stream();
 void upload_table(void* dst, const void* src, size_t bytes);
