@@ -74,10 +74,6 @@ __device__ __forceinline__ C2 ld_c2(const float4* p) {  // shared or global memo
   const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(p);
   return {v.x, v.y};
 }
-__device__ __forceinline__ C2 ldg_c2(const float4* p) {
-  const ulonglong2 v = __ldg(reinterpret_cast<const ulonglong2*>(p));
-  return {v.x, v.y};
-}
 __device__ __forceinline__ void st_c2(float4* p, C2 v) { *reinterpret_cast<ulonglong2*>(p) = make_ulonglong2(v.r, v.i); }
 
 // ---------------------------------------------------------------------------------------

@@ -78,16 +78,20 @@ __device__ __forceinline__ void copy_table(float4* dst, const float4* __restrict
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = __ldg(src + i);
 }
 __device__ __forceinline__ C2 wide(float2 w) { return {pk(w.x, w.x), pk(w.y, w.y)}; }
-__device__ __forceinline__ C2 ldg_c2_early(const float4* p) {  // not moved across other such loads
+__device__ __forceinline__ float2 table_root(const float2* __restrict__ p) { return __ldg(p); }
+__device__ __forceinline__ C2 ld_c2_early(const float4* p) {  // not moved across other loads
   C2 v;
-  asm volatile("ld.global.nc.v2.u64 {%0, %1}, [%2];" : "=l"(v.r), "=l"(v.i) : "l"(p));
+  asm volatile("ld.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.r), "=l"(v.i) : "l"(p) : "memory");
   return v;
 }
-
 
 // The three passes are launched so that a pass may start before the one ahead of it in the stream has
 // finished (launch_after): each lets the next one start at once, copies its tables, which no pass
 // writes, and waits here for the passes ahead to complete before it reads or writes anything else.
+// What a pass ahead may have written (psi, q, the tiles' and the kernel's spectra) is read by ordinary
+// loads: the read-only path (__ldg, ld.global.nc, const __restrict__ parameters) asks for memory that
+// nothing writes while the kernel lives, and its life begins before that wait.  Both measure the same
+// (4 views, a first call: 10 iterations of 512x512x256 77.9 ms, 20 of 256x256x192 30.9 ms).
 __device__ __forceinline__ void let_next_start() { cudaTriggerProgrammaticLaunchCompletion(); }
 __device__ __forceinline__ void wait_for_passes_ahead() { cudaGridDependencySynchronize(); }
 
@@ -129,9 +133,9 @@ struct PairRows<GatherMirror> {
   }
   __device__ __forceinline__ const float* row(int gy) const { return slice + (long long)reflect(gy, ny) * nx; }
   __device__ __forceinline__ int col(int gx) const { return reflect(gx, nx); }
-  __device__ __forceinline__ float load(const float* r, int c) const { return __ldg(r + c); }
+  __device__ __forceinline__ float load(const float* r, int c) const { return r[c]; }
   __device__ __forceinline__ float2 load2(const float* r, int gx) const {
-    return __ldg(reinterpret_cast<const float2*>(r + gx));
+    return *reinterpret_cast<const float2*>(r + gx);
   }
 };
 
@@ -147,9 +151,9 @@ struct PairRows<GatherValue> {
     return gy >= y0 && gy < y1 ? slice + (long long)gy * nx : nullptr;
   }
   __device__ __forceinline__ int col(int gx) const { return gx >= x0 && gx < x1 ? gx : -1; }
-  __device__ __forceinline__ float load(const float* r, int c) const { return r && c >= 0 ? __ldg(r + c) : value; }
+  __device__ __forceinline__ float load(const float* r, int c) const { return r && c >= 0 ? r[c] : value; }
   __device__ __forceinline__ float2 load2(const float* r, int gx) const {
-    return r ? __ldg(reinterpret_cast<const float2*>(r + gx)) : make_float2(value, value);
+    return r ? *reinterpret_cast<const float2*>(r + gx) : make_float2(value, value);
   }
 };
 
@@ -368,7 +372,7 @@ pair_fwd(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ sp
 // ------------------------------------------------------------------------------------------
 // y stage 1 inverse: a column pair of the spectrum slice to row pairs of columns c and c + pc
 template <int R>
-__device__ __forceinline__ void pair_y1_inv(const PairShape& s, const float4* __restrict__ in, float4* sm) {
+__device__ __forceinline__ void pair_y1_inv(const PairShape& s, const float4* in, float4* sm) {
   const int nb = s.pc * s.r0y, T = blockDim.x;
   int k0 = threadIdx.x / s.pc, c = threadIdx.x - k0 * s.pc;
   const int dk = T / s.pc, dc = T - dk * s.pc;
@@ -376,7 +380,7 @@ __device__ __forceinline__ void pair_y1_inv(const PairShape& s, const float4* __
     const float4* p = in + (k0 * R) * s.pc + c;
     C2 v[R];
 #pragma unroll
-    for (int r = 0; r < R; ++r) v[r] = ldg_c2(p + r * s.pc);
+    for (int r = 0; r < R; ++r) v[r] = ld_c2(p + r * s.pc);
     PDft<R, true>::run(v);
     const float2* w = reinterpret_cast<const float2*>(s.tab + s.tab_y) + k0 * R;
     float4* o = sm + (k0 * (R / 2)) * s.pitch + c;
@@ -387,7 +391,7 @@ __device__ __forceinline__ void pair_y1_inv(const PairShape& s, const float4* __
       unpk(v[2 * h].i, ai, bi);
       unpk(v[2 * h + 1].r, cr, dr);
       unpk(v[2 * h + 1].i, ci, di);
-      const float2 t = __ldg(w + 2 * h + 1);
+      const float2 t = table_root(w + 2 * h + 1);
       float4 A, B;
       if (h == 0) {
         A.x = ar;
@@ -395,7 +399,7 @@ __device__ __forceinline__ void pair_y1_inv(const PairShape& s, const float4* __
         B.x = br;
         B.z = bi;
       } else {
-        const float2 t0 = __ldg(w + 2 * h);
+        const float2 t0 = table_root(w + 2 * h);
         A.x = ar * t0.x + ai * t0.y;
         A.z = ai * t0.x - ar * t0.y;
         B.x = br * t0.x + bi * t0.y;
@@ -587,7 +591,7 @@ struct PairEpi {
 // Items: slices [hz, hz + ez of the first tile) of every tile; a tile clipped along z has fewer.
 template <class Epi>
 __global__ void __launch_bounds__(kPairThreads, 1)
-pair_inv(const TileDesc* __restrict__ tiles, int ntiles, const float4* __restrict__ spec, Epi epi,
+pair_inv(const TileDesc* __restrict__ tiles, int ntiles, const float4* spec, Epi epi,
          const __grid_constant__ PairShape s) {
   extern __shared__ float4 sm4[];
   float4* const sm = sm4;
@@ -655,7 +659,7 @@ pair_inv(const TileDesc* __restrict__ tiles, int ntiles, const float4* __restric
 // CONV: forward, times the kernel spectrum, inverse (effective slices stored); else forward, scaled
 // (kernel spectra).
 template <int R>
-__device__ __forceinline__ void pair_za_fwd(const PairShape& s, const float4* __restrict__ g, int plane, int count,
+__device__ __forceinline__ void pair_za_fwd(const PairShape& s, const float4* g, int plane, int count,
                                             float4* sm) {
   const int NR = s.bz * s.cz, nb = NR * kPairChunk;
   for (int b = threadIdx.x; b < nb; b += blockDim.x) {
@@ -698,14 +702,14 @@ __device__ __forceinline__ void pair_zb(const PairShape& s, float4* sm, const fl
 }
 
 template <int R, bool CONV>
-__device__ __forceinline__ void pair_zc(const PairShape& s, float4* __restrict__ g, const float4* __restrict__ otf,
+__device__ __forceinline__ void pair_zc(const PairShape& s, float4* __restrict__ g, const float4* otf,
                                         int plane, int count, float4* sm, float scale, const float2* tw) {
   const int nb = s.az * s.bz * kPairChunk, i = threadIdx.x % kPairChunk;
   C2 o[R];
   auto load = [&](int b) {
     if (CONV && b < nb && i < count) {
 #pragma unroll
-      for (int m = 0; m < R; ++m) o[m] = ldg_c2_early(otf + ((b / kPairChunk) * R + m) * plane + i);
+      for (int m = 0; m < R; ++m) o[m] = ld_c2_early(otf + ((b / kPairChunk) * R + m) * plane + i);
     }
   };
   int b = threadIdx.x;
@@ -768,7 +772,7 @@ __device__ __forceinline__ void pair_za_inv(const PairShape& s, float4* __restri
 // kernel spectrum is read from L2 by every tile but the first.
 template <bool CONV>
 __global__ void __launch_bounds__(kPairZThreads, 4)
-pair_z(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ spec, const float4* __restrict__ otf,
+pair_z(const TileDesc* __restrict__ tiles, int ntiles, float4* __restrict__ spec, const float4* otf,
        const __grid_constant__ PairShape s, int nchunks, int block, float scale) {
   extern __shared__ float4 sm4[];
   float4* const sm = sm4;
