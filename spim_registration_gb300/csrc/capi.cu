@@ -780,7 +780,10 @@ std::unique_ptr<ConvPlan> plan_view(mvd_decon* h, int v, const int lo[3], const 
       } catch (const std::invalid_argument&) {
         continue;
       }
-      if (!p->paired) continue;  // no pair shape within this budget
+      if (!p->paired) {
+        if (kb == 0) break;  // none at all, or the scalar kernels are the faster ones: time those
+        continue;            // no pair shape within this budget
+      }
       const std::array<int, 3> shape{p->ax.T, p->ay.T, p->az.T};
       if (std::find(seen.begin(), seen.end(), shape) != seen.end()) continue;
       seen.push_back(shape);
@@ -810,7 +813,13 @@ std::unique_ptr<ConvPlan> plan_view(mvd_decon* h, int v, const int lo[3], const 
   float best_ms = 1e30f;
   seen.clear();
   for (int cap : {4608, 7168, 10240, 14336}) {
-    auto p = make(cap, false);
+    std::unique_ptr<ConvPlan> p;
+    try {
+      p = make(cap, false);
+    } catch (const std::invalid_argument&) {
+      if (cap == 14336 && !best) throw;  // the kernel is too large for every budget
+      continue;
+    }
     const std::array<int, 3> shape{p->ax.T, p->ay.T, p->az.T};
     if (std::find(seen.begin(), seen.end(), shape) != seen.end()) continue;
     seen.push_back(shape);

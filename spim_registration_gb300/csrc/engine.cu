@@ -763,23 +763,9 @@ void ConvPlan::upload_pair() {
   ps.perz = ps.bz > 1 ? ps.bz : ps.az;
 }
 
-std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, int kx, int ky,
-                                         int kz, const PlanOptions& opt) {
-  if (nx < 1 || ny < 1 || nz < 1) throw std::invalid_argument("empty volume");
-  if (kx < 1 || ky < 1 || kz < 1 || !(kx & 1) || !(ky & 1) || !(kz & 1))
-    throw std::invalid_argument("kernel sizes must be odd and positive");
-  if (use_pairs() && !opt.scalar) {
-    auto plan = std::make_unique<ConvPlan>();
-    ConvPlan& p = *plan;
-    p.nx = nx; p.ny = ny; p.nz = nz;
-    p.kx = kx; p.ky = ky; p.kz = kz;
-    p.vol[0] = nx; p.vol[1] = ny; p.vol[2] = nz;
-    p.box_hi[0] = nx; p.box_hi[1] = ny; p.box_hi[2] = nz;
-    if (plan_pairs(p, nx, ny, nz, kx, ky, kz, opt)) {
-      p.upload();
-      return plan;
-    }
-  }
+// Tile shape of the scalar kernels; false when none fits the kernel.
+static bool scalar_tiles(int nx, int ny, int nz, int kx, int ky, int kz, const PlanOptions& opt, AxisTiles& bx,
+                         AxisTiles& by, AxisTiles& bz) {
   auto opts = [&](int size, int k, bool even, int tmax, int force) {
     if (force > 0) {
       AxisTiles a;
@@ -798,7 +784,6 @@ std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, 
   auto oy = opts(ny, ky, false, kPlaneCap / 2, opt.force_ty);
   auto oz = opts(nz, kz, false, kPlaneCap / kZPitch, opt.force_tz);
   double best = 1e300;
-  AxisTiles bx, by, bz;
   // an explicit budget (the autotuner's candidates) is a hard limit; the default plan weighs
   // the plane size and the compiled shapes (plane_cost_factor)
   const int limit = opt.cap > 0 ? opt.cap : plane_limit();
@@ -818,7 +803,49 @@ std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, 
         }
       }
     }
-  if (best >= 1e300) throw std::invalid_argument("no tile shape fits this kernel (kernel too large)");
+  return best < 1e300;
+}
+
+// Whether the scalar kernels are the faster ones although the pair kernels have a shape: their lengths
+// reach further along an axis (the pair kernels' end at 512, 200 and 400 points in x, y and z), so a
+// kernel nearly as long as those leaves a pair plan many tiles that are mostly halo.  The time of an
+// iteration goes with the padded voxels, of which a scalar pass takes about 2.4 times as long: scalar /
+// pair time against pair / scalar padding, at volumes from 128x128x64 to 512x512x256 and kernels of 121 to
+// 501 points along one axis: 1.3 to 1.6 at 1.4 to 1.8, 1.03 to 1.13 at 2.1 to 2.5, 0.7 to 0.9 at 2.6 to
+// 3.1, 0.2 at 12 (21x161x21 on 400x300x200: 2.23 ms on pairs, 2.30 scalar; 21x175x21: 3.25, 2.30; 15x195x15
+// on 256x256x192: 5.98, 1.16).  With no more planes than SMs a pass is one plane's latency, and the pair
+// kernels win at any padding (31x31x1 on 64x64x1: 41 us with 38 times the volume, 58).
+constexpr double kScalarPaddingCost = 2.4;
+static bool scalar_plan_pays(const ConvPlan& p) {
+  if ((long long)p.tiles.size() * p.ps.tz <= 152) return false;
+  const double most = (double)p.padded_voxels() / kScalarPaddingCost;
+  // no plan pads to less than one tile of the exact size
+  if (most <= (double)(p.nx + p.kx - 1) * (p.ny + p.ky - 1) * (p.nz + p.kz - 1)) return false;
+  AxisTiles x, y, z;
+  if (!scalar_tiles(p.nx, p.ny, p.nz, p.kx, p.ky, p.kz, PlanOptions(), x, y, z)) return false;
+  return (double)x.n * x.T * y.n * y.T * z.n * z.T < most;
+}
+
+std::unique_ptr<ConvPlan> make_conv_plan(PlanTable& pt, int nx, int ny, int nz, int kx, int ky,
+                                         int kz, const PlanOptions& opt) {
+  if (nx < 1 || ny < 1 || nz < 1) throw std::invalid_argument("empty volume");
+  if (kx < 1 || ky < 1 || kz < 1 || !(kx & 1) || !(ky & 1) || !(kz & 1))
+    throw std::invalid_argument("kernel sizes must be odd and positive");
+  if (use_pairs() && !opt.scalar) {
+    auto plan = std::make_unique<ConvPlan>();
+    ConvPlan& p = *plan;
+    p.nx = nx; p.ny = ny; p.nz = nz;
+    p.kx = kx; p.ky = ky; p.kz = kz;
+    p.vol[0] = nx; p.vol[1] = ny; p.vol[2] = nz;
+    p.box_hi[0] = nx; p.box_hi[1] = ny; p.box_hi[2] = nz;
+    if (plan_pairs(p, nx, ny, nz, kx, ky, kz, opt) && !scalar_plan_pays(p)) {
+      p.upload();
+      return plan;
+    }
+  }
+  AxisTiles bx, by, bz;
+  if (!scalar_tiles(nx, ny, nz, kx, ky, kz, opt, bx, by, bz))
+    throw std::invalid_argument("no tile shape fits this kernel (kernel too large)");
   auto plan = std::make_unique<ConvPlan>();
   ConvPlan& p = *plan;
   p.nx = nx; p.ny = ny; p.nz = nz;

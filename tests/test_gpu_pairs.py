@@ -9,7 +9,7 @@ import numpy as np
 import pytest
 
 from oracle import mvdecon_oracle as O
-from spim_registration_gb300 import Deconvolution, native
+from spim_registration_gb300 import FLAG_AUTOTUNE, Deconvolution, native
 from spim_registration_gb300 import synthetic as S
 from tests.helpers import rel_l2, rel_max
 
@@ -92,3 +92,31 @@ def test_deconvolution_of_boxes_matches_fp64(shape, lo, hi):
             _, _, rs, rm = [x for x in od.stats if x[0] == p.iterations - 1 and x[1] == v][0]
             assert s == pytest.approx(rs, rel=1e-3)
             assert m == pytest.approx(rm, rel=1e-3, abs=1e-6)
+
+
+@pytest.mark.parametrize("shape,kshape,paired", [
+    ((64, 128, 128), (15, 195, 15), False),   # 12 times the padding of the scalar lengths
+    ((91, 157, 203), (21, 171, 21), False),   # 2.8 times
+    ((91, 157, 203), (21, 141, 21), True),    # 1.9 times
+    ((91, 157, 203), (381, 21, 21), False),
+    ((91, 157, 203), (21, 21, 481), False),
+    ((1, 64, 64), (1, 31, 31), True),         # fewer planes than SMs: any padding
+])
+def test_kernels_near_the_longest_lengths_take_the_cheaper_plan(shape, kshape, paired):
+    """Kernels so long that a pair plan's tiles would be mostly halo run the scalar kernels, whose
+    lengths reach further, and either way the convolution is the oracle's."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(kshape[1])
+    x = (rng.random(shape) * 100 + 1).astype(np.float32)
+    k = rng.random(kshape).astype(np.float32)
+    k /= k.sum()
+    for flags in (0, FLAG_AUTOTUNE):
+        with Deconvolution([x], [np.ones(shape, np.float32)], [k], S.INDEPENDENT, 0.0, 0, flags) as d:
+            plan = d.plan(0)
+        assert (plan["kernels"] == "paired") == paired, plan
+    xd, kd = torch.from_numpy(x).cuda(), torch.from_numpy(k).cuda()
+    out = torch.full_like(xd, float("nan"))
+    torch.cuda.synchronize()
+    native.check(native.load().mvd_convolve3d_device(xd.data_ptr(), out.data_ptr(), native.iarr(shape[::-1]),
+                                                     kd.data_ptr(), native.iarr(kshape[::-1]), 0, 0.0, 0, None))
+    assert rel_max(out.cpu().numpy(), O.conv_extended(x, k, O.MIRROR, 0.0)) < TOL
