@@ -23,8 +23,9 @@ __global__ void cross_accumulate_kernel(const float2* __restrict__ B, const floa
   }
 }
 
-void dev_cross_accumulate(const float2* B, const float2* A, int ntiles, long long elems, float2* acc, cudaStream_t s) {
-  cross_accumulate_kernel<<<grid1(elems), 256, 0, s>>>(B, A, ntiles, elems, acc);
+void dev_cross_accumulate(const ConvPlan& p, const float2* B, const float2* A, float2* acc, cudaStream_t s) {
+  require_scalar(p, "the cross-spectrum sum");
+  cross_accumulate_kernel<<<grid1(p.otf_elems), 256, 0, s>>>(B, A, (int)p.tiles.size(), p.otf_elems, acc);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -1417,7 +1417,7 @@ extern "C" int mvd_backward(mvd_decon* h, float* grad_psi, float* const* grad_ps
     launch_z_forward(h->pt, p, TileSet::All, sa, 1.f, s);
     launch_fwd_masked(h->pt, p, h->r.as<float>(), sb, s);
     launch_z_forward(h->pt, p, TileSet::All, sb, 1.f, s);
-    dev_cross_accumulate(sb, sa, (int)p.tiles.size(), p.otf_elems, h->acc.as<float2>(), s);
+    dev_cross_accumulate(p, sb, sa, h->acc.as<float2>(), s);
     launch_z_inverse(h->pt, p, TileSet::Full, h->acc.as<float2>(), s);
     launch_inv_store_tiles(h->pt, p, TileSet::Full, h->acc.as<float2>(), h->lag_real.as<float>(), p.ax.T, p.ay.T, s);
     const double n_tile = (double)p.ax.T * p.ay.T * p.az.T;

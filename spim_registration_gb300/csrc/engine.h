@@ -296,19 +296,24 @@ long long launch_count();
 void count_launch(int n = 1);
 
 // ---- forward/backward of the Poisson image-formation model (adjoint.cu, passes_*.cu) ----
-// (the PSF gradient's passes take scalar plans only)
+// The PSF gradient's passes exist for scalar plans only: on a pair plan's tables and spectrum order they
+// would give wrong numbers or write past a buffer, so they throw.
+inline void require_scalar(const ConvPlan& p, const char* pass) {
+  if (p.paired) throw std::logic_error(std::string(pass) + " takes scalar plans only");
+}
 // forward plane pass of `vol` (value 0 outside) keeping only each tile's effective region
 void launch_fwd_masked(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s);
 // inverse-only z pass
 void launch_z_inverse(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, cudaStream_t s);
-// inverse plane pass storing the effective region of the tiles into out (dims nx, ny)
+// inverse plane pass storing the effective region of the tiles into out (dims nx, ny); pair plans: all
+// tiles only
 void launch_inv_store_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float2* spec, float* out, int nx,
                             int ny, cudaStream_t s);
 // inverse plane pass with the NLL epilogue: nll += sum, r = residual (r may be null)
 void launch_inv_nll(PlanTable& pt, const ConvPlan& p, const float2* spec, const float* img, const float* w, float* r,
                     double* nll, cudaStream_t s);
-// acc[i] = sum_t B_t[i] conj(A_t[i]) over `ntiles` tile spectra of `elems` values each (scalar plans)
-void dev_cross_accumulate(const float2* B, const float2* A, int ntiles, long long elems, float2* acc, cudaStream_t s);
+// acc[i] = sum_t B_t[i] conj(A_t[i]) over the spectra of p's tiles
+void dev_cross_accumulate(const ConvPlan& p, const float2* B, const float2* A, float2* acc, cudaStream_t s);
 // the factor by which the forward passes of p scale a spectrum (2 for the pair kernels)
 inline double spectrum_scale(const ConvPlan& p) { return p.paired ? 2.0 : 1.0; }
 

@@ -153,6 +153,7 @@ void launch_fwd_value_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const
 }
 
 void launch_fwd_masked(PlanTable& pt, const ConvPlan& p, const float* vol, float2* spec, cudaStream_t s) {
+  require_scalar(p, "the masked forward pass");
   GatherValue g = GatherValue::full(vol, p.vol[0], p.vol[1], p.vol[2], 0.f);
   launch_fwd_impl<GatherValue, true>(pt, p.d_tiles.as<TileDesc>(), p.d_items_fwd.as<int2>(), (int)p.items_fwd.size(),
                                      p.smem_plane, p.threads_plane, p.ax.T, p.ay.T, spec, g, s);

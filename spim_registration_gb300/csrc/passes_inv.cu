@@ -100,8 +100,9 @@ void launch_inv_nll(PlanTable& pt, const ConvPlan& p, const float2* spec, const 
 
 void launch_inv_store_tiles(PlanTable& pt, const ConvPlan& p, TileSet set, const float2* spec, float* out, int nx,
                             int ny, cudaStream_t s) {
-  if (p.paired) return pair_inv_store(p, spec, EpiStore{out, nx, ny}, s);  // TileSet::All
   const bool all = set == TileSet::All;
+  if (!all) require_scalar(p, "the inverse plane pass of one full tile");
+  if (p.paired) return pair_inv_store(p, spec, EpiStore{out, nx, ny}, s);
   const TileDesc* tiles = (all ? p.d_tiles : p.d_otf_tile).as<TileDesc>();
   const int2* items = (all ? p.d_items_inv : p.d_otf_fwd).as<int2>();  // the full tile: every slice
   const int nitems = all ? (int)p.items_inv.size() : p.n_otf_fwd;

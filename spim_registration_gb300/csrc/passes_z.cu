@@ -190,6 +190,7 @@ void launch_z_forward(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spe
 }
 
 void launch_z_inverse(PlanTable& pt, const ConvPlan& p, TileSet set, float2* spec, cudaStream_t s) {
+  require_scalar(p, "the inverse z pass");
   const bool all = set == TileSet::All;
   const int nitems = all ? (int)p.items_z.size() : p.n_otf_z;
   if (nitems == 0) return;
