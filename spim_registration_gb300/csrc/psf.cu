@@ -8,7 +8,6 @@
 
 #include <algorithm>
 #include <cfloat>
-#include <climits>
 #include <cmath>
 #include <string>
 
@@ -98,7 +97,7 @@ __device__ __forceinline__ float lerp(float a, float v0, float v1) {
 __global__ void __launch_bounds__(kExtractThreads, 4) extract_partial_kernel(
     const float* __restrict__ img, int sx, int sy, int sz, const Bead* __restrict__ beads, int n, int per, int px,
     int py, int pz, int xb, int yb, int items, float* __restrict__ part) {
-  const int item = (blockIdx.x * kExtractThreads + threadIdx.x) >> 5;
+  const int item = blockIdx.x * (kExtractThreads / 32) + (threadIdx.x >> 5);
   if (item >= items) return;
   const int x = (item % xb) * 32 + (threadIdx.x & 31);
   const int y0 = (item / xb) % yb * kRunY, z0 = item / (xb * yb) * kRunZ;
@@ -313,12 +312,8 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
     MVD_CHECK(cudaSetDevice(devCUDA));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int xb = (psf_dims[0] + 31) / 32, yb = (psf_dims[1] + kRunY - 1) / kRunY;
-    const long long items_ll = (long long)xb * yb * ((psf_dims[2] + kRunZ - 1) / kRunZ);
-    if (items_ll * 32 > INT_MAX) {
-      set_last_error("PSF too large");
-      return MVD_ERR_ARG;
-    }
-    const int items = (int)items_ll;
+    // warps: at most the PSF's voxels (2^30), though their threads may be more than an int holds
+    const int items = xb * yb * ((psf_dims[2] + kRunZ - 1) / kRunZ);
     // chunks of beads: about 24 warps per SM in all, partial sums of at most 256 MB
     const long long want = std::min((152LL * 24 + items - 1) / items, std::max(1LL, (64LL << 20) / np));
     const int per = (int)std::max(1LL, (num_locations + want - 1) / want);
@@ -344,7 +339,8 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
       MVD_CHECK(cudaGetLastError());
       count_launch();
     }
-    extract_partial_kernel<<<dim3((items * 32 + kExtractThreads - 1) / kExtractThreads, chunks), kExtractThreads, 0, s>>>(
+    constexpr int kWarps = kExtractThreads / 32;
+    extract_partial_kernel<<<dim3((items + kWarps - 1) / kWarps, chunks), kExtractThreads, 0, s>>>(
         img, dims[0], dims[1], dims[2], d_beads, num_locations, per, psf_dims[0], psf_dims[1], psf_dims[2], xb, yb, items,
         d_part);
     MVD_CHECK(cudaGetLastError());

@@ -139,3 +139,17 @@ def test_extraction_is_done_with_pageable_locations_on_return():
         mine[...] = np.nan
     torch.cuda.synchronize()
     assert torch.equal(outs[0], outs[1]) and torch.isfinite(outs[0]).all()
+
+
+def test_extraction_of_a_thin_psf_of_many_voxels():
+    """A PSF whose runs of 32 lanes hold more threads than an int counts: one voxel per lane's row, each the
+    periodic view's own value (a bead on a voxel centre)."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 28
+    img = torch.arange(1, 31, dtype=torch.float32, device="cuda").view(1, 30, 1)
+    locs = np.array([[0.0, 11.0, 0.0]])
+    out = torch.empty((1, n, 1), device="cuda")
+    s = torch.cuda.current_stream()
+    _extract_on(native.load(), torch, img, locs.ctypes.data, 1, (1, n, 1), out, s)
+    y = (torch.arange(n, device="cuda") - n // 2 + 11) % 30
+    assert torch.equal(out.view(-1), (y + 1).float())
