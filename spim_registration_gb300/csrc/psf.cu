@@ -70,12 +70,14 @@ __global__ void split_beads_kernel(const double* __restrict__ locations, int n, 
   beads[l] = Bead{base[0], base[1], base[2], frac[0], frac[1], frac[2]};
 }
 
-__device__ __forceinline__ int wrap(int i, int n) {  // i >= 0; one subtraction unless the PSF is larger than the view
+// Position i of an axis of n voxels repeated; one subtraction unless the PSF is larger than the view.
+// Unsigned: a base below 2^31 plus a position in the PSF may pass 2^31.
+__device__ __forceinline__ int wrap(unsigned i, unsigned n) {
   if (i >= n) {
     i -= n;
     if (i >= n) i %= n;
   }
-  return i;
+  return (int)i;
 }
 
 constexpr int kRunY = 4, kRunZ = 8;  // PSF voxels of a thread: 4 x 8 at one x, lanes along x
@@ -109,14 +111,14 @@ __global__ void __launch_bounds__(kExtractThreads, 4) extract_partial_kernel(
   const int l1 = min(n, ((int)blockIdx.y + 1) * per);
   for (int l = blockIdx.y * per; l < l1; ++l) {
     const Bead b = beads[l];
-    const int x0 = wrap(b.x + x, sx), x1 = wrap(b.x + x + 1, sx);
+    const int x0 = wrap((unsigned)b.x + x, sx), x1 = wrap((unsigned)b.x + x + 1, sx);
     int row[kRunY + 1];
 #pragma unroll
-    for (int y = 0; y <= kRunY; ++y) row[y] = wrap(b.y + y0 + y, sy);
+    for (int y = 0; y <= kRunY; ++y) row[y] = wrap((unsigned)b.y + y0 + y, sy);
     float last[kRunY];
 #pragma unroll
     for (int k = 0; k <= kRunZ; ++k) {
-      const float* slice = img + (long long)wrap(b.z + z0 + k, sz) * sy * sx;
+      const float* slice = img + (long long)wrap((unsigned)b.z + z0 + k, sz) * sy * sx;
       float t[kRunY + 1];
 #pragma unroll
       for (int y = 0; y <= kRunY; ++y) {

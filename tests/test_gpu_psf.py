@@ -153,3 +153,19 @@ def test_extraction_of_a_thin_psf_of_many_voxels():
     _extract_on(native.load(), torch, img, locs.ctypes.data, 1, (1, n, 1), out, s)
     y = (torch.arange(n, device="cuda") - n // 2 + 11) % 30
     assert torch.equal(out.view(-1), (y + 1).float())
+
+
+def test_extraction_at_the_end_of_an_axis_near_2_to_the_31():
+    """Positions in the PSF pass 2^31 before they wrap to the view's start."""
+    torch = pytest.importorskip("torch")
+    nx = 2**31 - 5
+    if torch.cuda.mem_get_info()[0] < 12 * 2**30:
+        pytest.skip("needs 9 GB")
+    img = torch.zeros((1, 1, nx), device="cuda")
+    img[0, 0, -20:] = torch.arange(1, 21, device="cuda")
+    img[0, 0, :20] = torch.arange(101, 121, device="cuda")
+    locs = np.array([[float(nx - 2), 0.0, 0.0]])
+    out = torch.empty((1, 1, 17), device="cuda")
+    _extract_on(native.load(), torch, img, locs.ctypes.data, 1, (17, 1, 1), out, torch.cuda.current_stream())
+    want = list(range(11, 21)) + list(range(101, 108))  # positions nx - 10 .. nx + 6
+    assert out.view(-1).tolist() == want
