@@ -1296,24 +1296,28 @@ void dev_paste_block(const float* block, int bx, int by, int bz, int lx, int ly,
   count_launch();
 }
 
-//
-// A warp takes a row of x at a time, four loads of each volume per lane in flight, so that y and z need
-// one division a row and one set of atomics a block.  A voxel per thread cost three 64-bit divisions at
-// every voxel with data: 73 us at 203x157x91 (23 MB).
+// A warp takes a row of x at a time (kBoxRun voxels of it, if it is longer), four loads of each volume per
+// lane in flight, so that y and z need one division a row and one set of atomics a block.  A voxel per
+// thread cost three 64-bit divisions at every voxel with data: 73 us at 203x157x91 (23 MB).  Rows
+// that one warp walked whatever their length took 546 us at 100000x300x1 (now 32).
+constexpr unsigned kBoxRun = 4096;
 __global__ void data_box_kernel(const float* __restrict__ img, const float* __restrict__ w, int nx, int ny, int nz,
                                 int* box) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   int lo[3] = {INT_MAX, INT_MAX, INT_MAX}, hi[3] = {-1, -1, -1};
-  const long long rows = (long long)ny * nz;
-  for (long long r = blockIdx.x * (long long)warps + warp; r < rows; r += (long long)gridDim.x * warps) {
+  const unsigned segs = ((unsigned)nx + kBoxRun - 1) / kBoxRun;
+  const long long items = (long long)ny * nz * segs;
+  for (long long i = blockIdx.x * (long long)warps + warp; i < items; i += (long long)gridDim.x * warps) {
+    const long long r = segs == 1 ? i : i / segs;
+    const unsigned xs = (unsigned)(i - r * segs) * kBoxRun, xe = min((unsigned)nx, xs + kBoxRun);
     const float* pi = img + r * nx;
     const float* pw = w + r * nx;
     bool any = false;
-    for (int x0 = lane; x0 < nx; x0 += 128) {
+    for (unsigned x0 = xs + lane; x0 < xe; x0 += 128) {  // unsigned: the last step may pass 2^31
       float a[4], b[4];
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
-        const bool in = x0 + 32 * e < nx;
+        const bool in = x0 + 32 * e < xe;
         a[e] = in ? __ldg(pi + x0 + 32 * e) : 0.f;
         b[e] = in ? __ldg(pw + x0 + 32 * e) : 0.f;
       }
@@ -1321,8 +1325,8 @@ __global__ void data_box_kernel(const float* __restrict__ img, const float* __re
       for (int e = 0; e < 4; ++e)
         if (a[e] > 0.f || b[e] > 0.f) {
           any = true;
-          lo[0] = min(lo[0], x0 + 32 * e);
-          hi[0] = max(hi[0], x0 + 32 * e);
+          lo[0] = min(lo[0], (int)(x0 + 32 * e));
+          hi[0] = max(hi[0], (int)(x0 + 32 * e));
         }
     }
     if (any) {
@@ -1354,7 +1358,8 @@ __global__ void data_box_kernel(const float* __restrict__ img, const float* __re
 }
 
 void dev_data_box(const float* img, const float* w, int nx, int ny, int nz, int* box, cudaStream_t s) {
-  const long long blocks = std::min(((long long)ny * nz + 7) / 8, 152LL * 8);  // one wave of 256 threads
+  const long long items = (long long)ny * nz * (((unsigned)nx + kBoxRun - 1) / kBoxRun);
+  const long long blocks = std::min((items + 7) / 8, 152LL * 8);  // one wave of 256 threads
   data_box_kernel<<<(int)blocks, 256, 0, s>>>(img, w, nx, ny, nz, box);
   MVD_CHECK(cudaGetLastError());
   count_launch();
