@@ -50,7 +50,7 @@ void dev_extract_lags(const float* R, int tx, int ty, int tz, int kx, int ky, in
 }
 
 // tab layout: [sx (nx+1) | ix | sy (ny+1) | iy | sz (nz+1) | iz] with the idx lengths nx+2hx etc.
-// A warp takes a row of x, so that y and z need one division a row.  An axis longer than the kernel's half
+// A warp takes a row of x, or `run` voxels of it, so that y and z need one division.  An axis longer than the kernel's half
 // has at most two positions per voxel; their up to eight values are all loaded before they are added, in
 // the order of the lists (one by one, each sum waited for the load before it: 71 us at 192^3, 31x31x61
 // kernel; now 43).
@@ -58,10 +58,13 @@ __global__ void __launch_bounds__(256) fold_mirror_kernel(const float* __restric
                                                           const int* __restrict__ sx, const int* __restrict__ ix,
                                                           const int* __restrict__ sy, const int* __restrict__ iy,
                                                           const int* __restrict__ sz, const int* __restrict__ iz,
-                                                          int nx, int ny, int nz, float* __restrict__ g) {
+                                                          int nx, int ny, int nz, int run, float* __restrict__ g) {
   const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const long long rows = (long long)ny * nz;
-  for (long long r = blockIdx.x * (long long)warps + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * warps) {
+  const int segs = (nx + run - 1) / run;
+  const long long items = (long long)ny * nz * segs;
+  for (long long i = blockIdx.x * (long long)warps + (threadIdx.x >> 5); i < items; i += (long long)gridDim.x * warps) {
+    const long long r = segs == 1 ? i : i / segs;
+    const int xs = (int)(i - r * segs) * run, xe = min(nx, xs + run);
     const int z = (int)(r / ny), y = (int)(r - (long long)z * ny);
     const int a0 = sz[z], a1 = sz[z + 1], b0 = sy[y], b1 = sy[y + 1];
     const bool two_a = a1 - a0 > 1, two_b = b1 - b0 > 1;
@@ -71,7 +74,7 @@ __global__ void __launch_bounds__(256) fold_mirror_kernel(const float* __restric
     const float* const r11 = two_a && two_b ? c + ((long long)iz[a0 + 1] * nye + iy[b0 + 1]) * nxe : nullptr;
     const bool few = a1 - a0 <= 2 && b1 - b0 <= 2;
 #pragma unroll 2
-    for (int x = lane; x < nx; x += 32) {
+    for (int x = xs + lane; x < xe; x += 32) {
       const int e0 = sx[x], e1 = sx[x + 1];
       const float old = g[r * nx + x];
       float acc = 0.f;
@@ -109,8 +112,14 @@ void dev_fold_mirror(const float* c, int nxe, int nye, const int* tab, int nx, i
   const int* iy = sy + ny + 1;
   const int* sz = iy + nye;
   const int* iz = sz + nz + 1;
-  const long long blocks = std::min(((long long)ny * nz + 7) / 8, 152LL * 32);
-  fold_mirror_kernel<<<(int)blocks, 256, 0, s>>>(c, nxe, nye, sx, ix, sy, iy, sz, iz, nx, ny, nz, g);
+  // whole rows where these are 64 warps per SM, else as many runs of at least 64 voxels: a row each took
+  // 8.7 ms at 100000x30x1, 3.3 ms at 20000x5x3 and 41 us at 2000x2000x1 (now 56, 20 and 25 us)
+  const long long rows = (long long)ny * nz;
+  const int segs = (int)std::max(1LL, std::min((152LL * 64 + rows - 1) / rows, (nx + 63LL) / 64));
+  const int run = ((nx + segs - 1) / segs + 31) / 32 * 32;
+  const long long items = rows * ((nx + run - 1) / run);
+  fold_mirror_kernel<<<(int)std::min((items + 7) / 8, 152LL * 32), 256, 0, s>>>(c, nxe, nye, sx, ix, sy, iy, sz, iz, nx,
+                                                                             ny, nz, run, g);
   MVD_CHECK(cudaGetLastError());
   count_launch();
 }

@@ -137,3 +137,14 @@ def test_set_kernel_is_complete_on_return():
             k[...] = -1.0
             assert idle
             np.testing.assert_array_equal(d.kernel(0, 1), want)
+
+
+def test_fold_of_few_long_rows_matches_oracle_gradient():
+    """Rows that several warps share, in runs that end inside the row (tolerance as above)."""
+    p = S.make_problem(5, shape_xyz=(333, 3, 2), psf_size_xyz=(9, 3, 3), n_blobs=10, n_views=2, iterations=1)
+    with Deconvolution(p.views, p.weights, p.psfs, p.psftype, p.lam) as d:
+        d.run(1)
+        psi = d.get_psi().astype(np.float64)
+        k1 = [d.kernel(v, 1).astype(np.float64) for v in range(2)]
+        g_psi, _ = d.backward()
+    assert rel_l2(g_psi, O.poisson_nll_grad(psi, p.views, p.weights, k1)[0]) < 1e-4
