@@ -51,23 +51,47 @@ struct Bead {
   float ax, ay, az;
 };
 
-// The beads of n locations (x, y, z triples), split in double (exactly): the device does it from the
-// caller's own array, so that a captured call has no host memory of its own that a replay would read.
-__global__ void split_beads_kernel(const double* __restrict__ locations, int n, int3 dims, int3 half,
-                                   Bead* __restrict__ beads) {
-  const int l = blockIdx.x * blockDim.x + threadIdx.x;
-  if (l >= n) return;
+// A location (x, y, z) split in double (exactly)
+__host__ __device__ inline Bead split_bead(const double* location, int3 dims, int3 half) {
   const int size[3] = {dims.x, dims.y, dims.z}, h[3] = {half.x, half.y, half.z};
   int base[3];
   float frac[3];
-#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const double t = locations[3LL * l + d], f = floor(t);
+    const double t = location[d], f = floor(t);
     frac[d] = (float)(t - f);  // NaN for a location that is not finite
     const double b = isfinite(t) ? fmod(f - (double)h[d], (double)size[d]) : 0.0;
     base[d] = (int)(b < 0.0 ? b + size[d] : b);
   }
-  beads[l] = Bead{base[0], base[1], base[2], frac[0], frac[1], frac[2]};
+  return Bead{base[0], base[1], base[2], frac[0], frac[1], frac[2]};
+}
+
+// The beads of n locations on the device.  A call passes up to kMostByValue beads as a kernel's
+// parameter, so that nothing of the caller's memory is read after it returns and nothing is waited for.
+// More beads, and those of a call under capture, are split on the device from a copy of the caller's own
+// array: a replay then reads that and no host memory of the call's.  4 views of 436 beads, 11x25x29 PSFs:
+// 653 to 671 us by value, 675 to 715 by a copy that is waited for.
+template <int N>
+struct BeadBlock {
+  Bead b[N];
+};
+constexpr int kMostByValue = 1360;  // 32640 of the 32764 bytes that a kernel's parameters may take
+template <int N>
+__global__ void store_beads_kernel(const __grid_constant__ BeadBlock<N> block, int n, Bead* __restrict__ beads) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < n) beads[l] = block.b[l];
+}
+__global__ void split_beads_kernel(const double* __restrict__ locations, int n, int3 dims, int3 half,
+                                   Bead* __restrict__ beads) {
+  const int l = blockIdx.x * blockDim.x + threadIdx.x;
+  if (l < n) beads[l] = split_bead(locations + 3LL * l, dims, half);
+}
+template <int N>
+void store_beads(const double* locations, int n, int3 dims, int3 half, Bead* beads, cudaStream_t s) {
+  BeadBlock<N> block;
+  for (int l = 0; l < n; ++l) block.b[l] = split_bead(locations + 3 * l, dims, half);
+  store_beads_kernel<N><<<(n + 127) / 128, 128, 0, s>>>(block, n, beads);
+  MVD_CHECK(cudaGetLastError());
+  count_launch();
 }
 
 // Position i of an axis of n voxels repeated; one subtraction unless the PSF is larger than the view.
@@ -321,23 +345,32 @@ extern "C" int mvd_extract_psf(const float* img, const int* dims, const double* 
     const int per = (int)std::max(1LL, (num_locations + want - 1) / want);
     const int chunks = std::max(1, (num_locations + per - 1) / per);
     const int nends = blocks_for(np);
-    const size_t lb = (size_t)num_locations * 3 * sizeof(double), bb = ((size_t)num_locations * sizeof(Bead) + 7) / 8 * 8,
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    MVD_CHECK(cudaStreamIsCapturing(s, &capture));
+    const bool by_value = capture == cudaStreamCaptureStatusNone && num_locations <= kMostByValue;
+    const size_t lb = by_value ? 0 : (size_t)num_locations * 3 * sizeof(double),
+                 bb = ((size_t)num_locations * sizeof(Bead) + 7) / 8 * 8,
                  eb = (size_t)nends * sizeof(float2);
     const CallBuf buf(devCUDA, lb + bb + eb + (size_t)chunks * np * sizeof(float), s);
     double* d_loc = buf.as<double>();
     Bead* d_beads = reinterpret_cast<Bead*>(buf.as<char>() + lb);
     float2* d_ends = reinterpret_cast<float2*>(buf.as<char>() + lb + bb);
     float* d_part = reinterpret_cast<float*>(buf.as<char>() + lb + bb + eb);
+    const int3 size = make_int3(dims[0], dims[1], dims[2]),
+               half = make_int3(psf_dims[0] / 2, psf_dims[1] / 2, psf_dims[2] / 2);
     // nothing of the caller's pageable memory is read once the call has returned
     CopyDone copied;
-    if (num_locations > 0) {
+    if (by_value) {
+      if (num_locations > 512)
+        store_beads<kMostByValue>(locations, num_locations, size, half, d_beads, s);
+      else if (num_locations > 160)
+        store_beads<512>(locations, num_locations, size, half, d_beads, s);
+      else if (num_locations > 0)
+        store_beads<160>(locations, num_locations, size, half, d_beads, s);
+    } else if (num_locations > 0) {
       MVD_CHECK(cudaMemcpyAsync(d_loc, locations, lb, cudaMemcpyHostToDevice, s));
-      cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-      MVD_CHECK(cudaStreamIsCapturing(s, &capture));
       if (capture == cudaStreamCaptureStatusNone && !async_copy_source(locations)) copied.record(s);
-      split_beads_kernel<<<(num_locations + 127) / 128, 128, 0, s>>>(
-          d_loc, num_locations, make_int3(dims[0], dims[1], dims[2]),
-          make_int3(psf_dims[0] / 2, psf_dims[1] / 2, psf_dims[2] / 2), d_beads);
+      split_beads_kernel<<<(num_locations + 127) / 128, 128, 0, s>>>(d_loc, num_locations, size, half, d_beads);
       MVD_CHECK(cudaGetLastError());
       count_launch();
     }

@@ -169,3 +169,22 @@ def test_extraction_at_the_end_of_an_axis_near_2_to_the_31():
     _extract_on(native.load(), torch, img, locs.ctypes.data, 1, (17, 1, 1), out, torch.cuda.current_stream())
     want = list(range(11, 21)) + list(range(101, 108))  # positions nx - 10 .. nx + 6
     assert out.view(-1).tolist() == want
+
+
+@pytest.mark.parametrize("beads", [160, 161, 512, 513, 1360, 1361])
+def test_beads_by_value_and_by_copy_match_oracle(beads):
+    """Bead counts on both sides of each size of the parameter block, and of the copy beyond them; the
+    array may be reused when the call returns."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(beads)
+    img = (rng.random((12, 14, 16)) * 100).astype(np.float32)
+    locs = rng.uniform(-20, 40, (beads, 3))
+    want = O.extract_psf_local(img, locs, (5, 3, 4))
+    d_img, out, s = torch.from_numpy(img).cuda(), torch.empty((4, 3, 5), device="cuda"), torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        torch.cuda._sleep(5_000_000)
+    _extract_on(native.load(), torch, d_img, locs.ctypes.data, beads, (5, 3, 4), out, s)
+    locs[...] = np.nan
+    s.synchronize()
+    _close(out.cpu().numpy(), want)
