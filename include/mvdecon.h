@@ -40,7 +40,8 @@ float* convolution3DfftCUDA(float* im, int* imDim, float* kernel, int* kernelDim
  * odd sizes, centre at size/2): true convolution of the block extended mirror-single at its
  * border, the result the CPU FFTConvolution gives on the same block.  Callers consume the
  * interior [k/2, dim - k/2).  Synchronous; no pointer is kept.  On failure `im` is left
- * unmodified and the reason is available from mvd_last_error(). */
+ * unmodified (unless what fails is the copy of the finished result into it) and the reason is
+ * available from mvd_last_error(). */
 void convolution3DfftCUDAInPlace(float* im, int* imDim, float* kernel, int* kernelDim, int devCUDA);
 
 /* ===================== Part 2: additions (status-returning) ===================== */
@@ -67,7 +68,8 @@ enum {
   MVD_FLAG_PLAIN = 1,    /* reference structure: one block per launch sequence, separate
                             quotient / update kernels, no graph (the plain FP32 GPU form) */
   MVD_FLAG_NO_GRAPH = 2, /* batched, fused passes but launched eagerly (no CUDA graph) */
-  MVD_FLAG_AUTOTUNE = 4, /* time candidate tile plans per view at creation and keep the fastest;
+  MVD_FLAG_AUTOTUNE = 4, /* time candidate tile plans per view at creation and keep the fastest
+                            (of the kind of kernels that the planner picks for the view);
                             the choice is kept for the process, so later handles with the same
                             data-box and kernel sizes on the same device reuse it untimed */
   MVD_FLAG_TENSOR_DFT = 8 /* z passes of the compiled pencil lengths 320 and 288 run their middle
@@ -230,7 +232,8 @@ int mvd_weight_overlap(const float* const* weights, int num_views, long long n, 
  * mvd_extract_psf: ExtractPSF.extractPSFLocal (:374-415): psf[p] = sum over the bead
  * locations (x, y, z triples, doubles, in the view's pixel frame; host array) of the view
  * (device, dims_xyz) interpolated trilinearly, extended periodically, at p - psf_dims / 2 +
- * location; locations are added in the given order.  normalize != 0 then applies
+ * location.  Chunks of the beads are summed in the given order, then the chunks' sums with the
+ * additions' errors carried along.  normalize != 0 then applies
  * ExtractPSF.normalize (:298-316): (v - min) / (max - min).  psf: device, overwritten.
  * A pageable locations array has been read when the call returns, a page-locked one when the stream
  * has passed the call.  A call on a stream under capture reads the array again at every replay. */

@@ -142,8 +142,8 @@ struct ConvPlan {
   bool ascending = false;              // radices of every length in ascending order
   bool generic = false;                // run the generic kernels even where a compiled shape exists
   bool staged = false;                 // large compiled planes: in-place kernels, two CTAs per SM
-  // the packed pair kernels (pair_kernels.cuh) run this plan; without them (a tile shape they do
-  // not have, or an option that asks for the scalar kernels) the item tables below are used
+  // the packed pair kernels (pair_kernels.cuh) run this plan; without them (no tile shape of theirs
+  // fits, the scalar kernels are faster, or an option asks for those) the item tables below are used
   bool paired = false;
   PairShape ps{};
   int pair_threads = 0;                // CTA size of the plane passes

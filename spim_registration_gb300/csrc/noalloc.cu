@@ -59,8 +59,8 @@ struct Axis {
   int T, n, E;
 };
 
-// tile choice: the allocating path's default rule (plane_limit, plane_cost_factor), so both
-// pick the same tiles
+// tile choice: the scalar planner's default rule (plane_limit, plane_cost_factor).  The allocating
+// path plans on the packed kernels, whose tiles are others.
 std::vector<Axis> options(int size, int k, bool even, int tmax) {
   std::vector<Axis> out;
   int last = -1;

@@ -1,4 +1,5 @@
-// Tiled FFT convolution passes on pairs of transforms (the default path of every convolution).
+// Tiled FFT convolution passes on pairs of transforms (the default path of every convolution whose
+// kernel is not nearly as long as their longest transforms).
 //
 // The three passes are those of kernels.cuh (forward planes, z pencils, inverse planes over
 // overlap-save tiles), rebuilt around packed FP32 arithmetic (pair_fft.cuh):
